@@ -68,7 +68,10 @@ enum nlm_decomposition {
   NLM_DECOMP_THREAD = 1,  /* one thread per node, sliced-ELL bonds taken
                              four at a time                                */
   NLM_DECOMP_WARP = 2,    /* one warp per node, CSR bond storage           */
-  NLM_DECOMP_THREAD1 = 3, /* one thread per node, one bond per iteration   */
+  NLM_DECOMP_THREAD1 = 3, /* one thread per node, one bond per iteration; in
+                             FP64: bond geometry recomputed every step instead
+                             of kept in HBM (68 bytes per 2-D bond), slower,
+                             same results                                  */
   NLM_DECOMP_TILE = 4,    /* FP32C 2-D RNPBond: 256-node tiles with their
                              halo staged in shared memory, 16-bit
                              tile-local bond ids                           */

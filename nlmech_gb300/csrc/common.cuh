@@ -29,6 +29,34 @@ inline bool dGT(double a, double b) { return (a - b) > (amax_d(a, b) * 1e-5); }
 inline bool dLT(double a, double b) { return (b - a) > (amax_d(a, b) * 1e-5); }
 #endif
 
+#ifdef __CUDACC__
+// Correctly rounded a / b from y = RN(1 / b): a first quotient, its exact
+// remainder, one correction (Markstein, IBM J. Res. Dev. 34 (1990) 111), 3
+// FP64 operations against the 9 or so of a division.  Differs from a / b
+// only where the remainder underflows or the quotient is not finite.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+// Loads of data read once per step: kept out of L1, which serves the gathers
+// of the neighbours' state.
+__device__ __forceinline__ double2 ld_once(const double2 *p) {
+  double2 v;
+  asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_once(const double *p) {
+  double v;
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_once(const int *p) {
+  int v;
+  asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+#endif
+
 // Node flag byte.
 enum : uint8_t {
   FLAG_FIX_X = 1,

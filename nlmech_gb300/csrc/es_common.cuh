@@ -13,11 +13,11 @@ __device__ __forceinline__ double es_omega(const StepParams &P, double Xl) {
   return dGT(Xl, P.delta - r) ? (P.delta + r - Xl) / P.h : 1.;
 }
 
-// Scalar force state t (ElasticState.cpp:191-245); e_d = e - e_s in 3-D unless
-// the reference's behaviour (e_d = 0) is requested.
+// Coefficients of the force state t (ElasticState.cpp:191-245) that a node's
+// m_i fixes: 2-D (2 f2 alpha_s - (3 - 2 f2) alpha_d, alpha_d), 3-D (alpha_s,
+// alpha_d).
 template <int DIM>
-__device__ __forceinline__ double es_t64(const StepParams &P, double mi, double theta, double e,
-                                         double Xl) {
+__device__ __forceinline__ double2 es_coef64(const StepParams &P, double mi) {
   if (DIM == 2) {
     double alpha_s;
     if (!P.es_plane_strain) {
@@ -27,20 +27,22 @@ __device__ __forceinline__ double es_t64(const StepParams &P, double mi, double 
       alpha_s = (9. / mi) * (P.es_K + P.es_mu / 9.);
     }
     const double alpha_d = (8. / mi) * P.es_mu;
-    const double e_s = theta * Xl / 3.;
-    const double e_d = e - e_s;
     const double f2 = P.es_factor2D;
-    const double t_s = (2. * f2 * alpha_s - (3. - 2. * f2) * alpha_d) * 1. * e_s / 3.;
-    const double t_d = alpha_d * 1. * e_d;
-    return t_s + t_d;
+    return make_double2((2. * f2 * alpha_s - (3. - 2. * f2) * alpha_d) * 1., alpha_d * 1.);
   }
-  const double alpha_s = (9. / mi) * P.es_K;
-  const double alpha_d = (15. / mi) * P.es_mu;
+  return make_double2((9. / mi) * P.es_K * 1., (15. / mi) * P.es_mu * 1.);
+}
+
+// Scalar force state t; e_d = e - e_s in 3-D unless the reference's behaviour
+// (e_d = 0) is requested.
+template <int DIM>
+__device__ __forceinline__ double es_t64(const StepParams &P, double mi, double theta, double e,
+                                         double Xl) {
+  const double2 c = es_coef64<DIM>(P, mi);
   const double e_s = theta * Xl / 3.;
-  const double e_d = P.es_ref_compat ? 0. : e - e_s;
-  const double t_s = alpha_s * 1. * e_s;
-  const double t_d = alpha_d * 1. * e_d;
-  return t_s + t_d;
+  const double e_d = DIM == 3 && P.es_ref_compat ? 0. : e - e_s;
+  const double t_s = DIM == 2 ? c.x * e_s / 3. : c.x * e_s;
+  return t_s + c.y * e_d;
 }
 
 template <int DIM>

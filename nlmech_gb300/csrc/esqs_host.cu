@@ -157,7 +157,7 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
     if (!(d.material.G > 0.)) d.material.G = 1.;
   }
   nlm_esqs *q = new nlm_esqs();
-  int rc = nlm_fd_create(&d, &q->fd);
+  int rc = create_model(&d, &q->fd, false);
   if (rc) {
     delete q;
     return rc;

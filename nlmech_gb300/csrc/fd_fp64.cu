@@ -6,10 +6,31 @@
 // node and sums its bonds in neighbour-list order (ascending original id), as
 // FDModel::computeForce does (src/model/fd/fDModel.cpp:557-575).
 
+#include <type_traits>
 #include "fd_internal.h"
 #include "state_io.cuh"
 
 namespace nlm {
+
+// exp(x): the Taylor polynomial of degree 7 where |x| < 2^-5 (bonds below a
+// quarter of the critical strain; truncation 2^-55, last operation a fused
+// 1 + x q, so within 0.53 ulp), CUDA's exp() elsewhere.  The polynomial is 7
+// FP64 instructions against about 19.
+constexpr int kExpSmall = 0x3fa00000;  // high word of 2^-5
+__device__ __forceinline__ double exp_small(double x) {
+  double q = 1. / 5040.;
+  q = __fma_rn(q, x, 1. / 720.);
+  q = __fma_rn(q, x, 1. / 120.);
+  q = __fma_rn(q, x, 1. / 24.);
+  q = __fma_rn(q, x, 1. / 6.);
+  q = __fma_rn(q, x, 0.5);
+  q = __fma_rn(q, x, 1.);
+  return __fma_rn(q, x, 1.);
+}
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+__device__ __forceinline__ double exp64(double x) {
+  return hi_abs(x) < kExpSmall ? exp_small(x) : exp(x);
+}
 
 // One RNPBond::getBondEF evaluation (src/material/pd/rnpBond.cpp:216-301),
 // contact force off.  Returns the scalar s of F = s * e and the unit vector e.
@@ -35,12 +56,26 @@ __device__ __forceinline__ double rnp_bond64(const StepParams &P, const double x
   if (breakable) {
     if (P.irrev && !fs && dGT(fabs(S), P.fsc * (P.rbar / sqrt(rji)))) fs = true;  // :263-266
     if (fs) return 0.0;
-    return (infl * 4. * S * P.C * P.beta * exp(-P.beta * rji * S * S) / P.invF) * volj;
+    return (infl * 4. * S * P.C * P.beta * exp64(-P.beta * rji * S * S) / P.invF) * volj;
   }
   return (infl * 4. * S * P.C * P.beta / P.invF) * volj;  // :298
 }
 
-// Thread-per-node step over the sliced-ELL bond store.
+// Normal contact of a broken bond (rnpBond.cpp:281-291): with y = (x_j + u_j)
+// - (x_i + u_i) the force is -max(0, Kn Vi Vj / (Vi + Vj) (Rc - |y|) / |y|) y;
+// returns the factor.
+__device__ __forceinline__ double contact64(const StepParams &P, const double xi[3],
+                                            const double ui[3], const double xj[3],
+                                            const double uj[3], double voli, double volj,
+                                            double y[3]) {
+  for (int c = 0; c < 3; c++) y[c] = (xj[c] + uj[c]) - (xi[c] + ui[c]);
+  const double R = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
+  const double sf = P.contact_kn * (voli * volj / (voli + volj)) * (P.contact_rc - R) / R;
+  return sf < 0. ? 0. : sf;
+}
+
+// Thread-per-node step over the sliced-ELL bond store, the bond's geometry
+// recomputed from the positions.
 template <int DIM, int SCHEME, bool FIRST>
 __global__ void __launch_bounds__(128)
     k_rnp64_thread(const StepParams P, const DevPtrs D, const BCTable T, const StepArgs A) {
@@ -85,13 +120,8 @@ __global__ void __launch_bounds__(128)
       fi[1] = fi[1] + s * e[1];
       if (DIM == 3) fi[2] = fi[2] + s * e[2];
     } else if (P.contact) {
-      // normal contact of a broken bond (rnpBond.cpp:281-291):
-      // y = (x_j + u_j) - (x_i + u_i), f += -max(0, Kn Vi Vj/(Vi+Vj) (Rc - |y|)/|y|) y
       double y[3];
-      for (int c = 0; c < 3; c++) y[c] = (xj[c] + uj[c]) - (xi[c] + ui[c]);
-      const double R = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
-      double sf = P.contact_kn * (voli * volj / (voli + volj)) * (P.contact_rc - R) / R;
-      if (sf < 0.) sf = 0.;
+      const double sf = contact64(P, xi, ui, xj, uj, voli, volj, y);
       fi[0] = fi[0] + (0. + -sf * y[0]);
       fi[1] = fi[1] + (0. + -sf * y[1]);
       if (DIM == 3) fi[2] = fi[2] + (0. + -sf * y[2]);
@@ -101,13 +131,205 @@ __global__ void __launch_bounds__(128)
   integrate_node64<DIM, SCHEME, FIRST>(P, D, T, A, i, fl, ui, fi);
 }
 
+// ---- step over the FP64 bond store ------------------------------------------
+// GB300 issues two FP64 lanes per SM and cycle, so an FP64 step is bound by
+// the number of FP64 instructions, not by memory: k_rnp64_thread spends about
+// 160 of them per bond, three quarters on what depends on the reference
+// geometry only (two square roots, four divisions, the volume factor).  The
+// bond store keeps those values (68 bytes per 2-D bond, read once per step in
+// 512-byte rows); every remaining operation is the reference's, rounded in
+// the same order, so the results are the same bits.
+// b64_thr: the high word of the break threshold S_c(r), below which |S| cannot
+// break the bond (one integer comparison instead of FP64 ones); bit 31 marks a
+// bond of a no-fail node, whose threshold is that of infinity.
+
+constexpr int kThrTough = (int)0x80000000u, kThrInf = 0x7ff00000;
+
+template <int DIM>
+__global__ void k_rnp64_store(const StepParams P, const DevPtrs D, double2 *bd, double2 *be,
+                              double2 *bz, double2 *bq, double2 *bm, double *bk, int *bt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  double xi[3];
+  ld_node<DIM>(D.pos64, i, xi);
+  const int64_t base = D.sell_ptr[i >> 5];
+  const int lane = (int)(i & 31), len = D.rowlen[i];
+  for (int k = 0; k < len; k++) {
+    const int j = D.sell_cols[base + 4 * lane + (k >> 2) * 128 + (k & 3)];
+    const int64_t q = base + 32 * (int64_t)k + lane;
+    double xj[3];
+    ld_node<DIM>(D.pos64, j, xj);
+    const double dx = xj[0] - xi[0], dy = xj[1] - xi[1], dz = DIM == 3 ? xj[2] - xi[2] : 0.;
+    double rr = dx * dx + dy * dy;
+    if (DIM == 3) rr = rr + dz * dz;
+    const double rji = sqrt(rr);
+    double volj = D.vol64[j];
+    if (dGT(rji, P.check_low)) volj = volj * ((P.check_up - rji) / P.h);
+    bd[q] = make_double2(dx, dy);
+    be[q] = make_double2(dx / rji, dy / rji);
+    if (DIM == 3) bz[q] = make_double2(dz, dz / rji);
+    bq[q] = make_double2(rr, __drcp_rn(rr));
+    bm[q] = make_double2(-P.beta * rji, volj);
+    if (bk) bk[q] = influence_d(P, rji / P.delta) * 4.;
+    int thr = kThrInf;
+    if ((D.flags[i] | D.flags[j]) & FLAG_NOFAIL)
+      thr |= kThrTough;
+    else if (P.irrev)
+      thr = max(0, min(kThrInf, __double2hiint(P.fsc * (P.rbar / sqrt(rji)))));
+    bt[q] = thr;
+  }
+}
+
+// G lanes share a node (G = 1: one thread per node); a lane takes U bonds of
+// each group of G * U, evaluated side by side to cover the FP64 latency, and
+// their contributions are added in row order.  Four bonds per lane take 139
+// registers and were slower (189 against 146 us), so are blocks of 128 (159).
+// 320 x 250 plate, horizon 3h: 605 us per step with k_rnp64_thread, 146 us
+// here, 33 FP64 instructions per bond, the FP64 pipe 85 % busy: the bound.
+template <int DIM, int SCHEME, bool FIRST, int G>
+__global__ void __launch_bounds__(128)
+    k_rnp64_bond(const StepParams P, const double inv_invF, const DevPtrs D, const BCTable T,
+                 const StepArgs A) {
+  constexpr int U = G == 16 ? 1 : 2, W = G * U;
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  if (i >= P.n) return;
+  const int c = threadIdx.x % G;
+  const unsigned team = G == 1 ? 0u : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G);
+  const double *ucur = D.u64[A.cur];
+  double ui[3];
+  ld_node<DIM>(ucur, i, ui);
+  const int64_t base = D.sell_ptr[i >> 5];
+  const int lane = (int)(i & 31), len = D.rowlen[i];
+  const int *colp = D.sell_cols + base + 4 * lane;
+  const double k0 = P.infl_a0 * 4.;
+  double fi[3] = {0., 0., 0.};
+  uint32_t word = 0;
+  for (int kb = 0; kb < len; kb += W) {
+    if ((kb & 31) == 0) word = D.bits[(int64_t)(kb >> 5) * P.npad + i];
+    double2 d[U], e[U], z[U], m[U];
+    double S[U], x[U], ex[U], uj[U][3], k4[U];
+    int thr[U], jj[U];
+    uint32_t add = 0, cut = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int k = min(kb + u * G + c, len - 1);
+      const int64_t q = base + 32 * (int64_t)k + lane;
+      jj[u] = __ldg(colp + (k >> 2) * 128 + (k & 3));
+      ld_node<DIM>(ucur, jj[u], uj[u]);
+      d[u] = ld_once(D.b64_d + q);
+      e[u] = ld_once(D.b64_e + q);
+      m[u] = ld_once(D.b64_m + q);
+      if (DIM == 3) z[u] = ld_once(D.b64_z + q);
+      thr[u] = ld_once(D.b64_thr + q);
+      k4[u] = D.b64_k ? ld_once(D.b64_k + q) : k0;
+      const double2 rq = ld_once(D.b64_q + q);
+      double dotp = d[u].x * (uj[u][0] - ui[0]) + d[u].y * (uj[u][1] - ui[1]);
+      if (DIM == 3) dotp = dotp + z[u].x * (uj[u][2] - ui[2]);
+      S[u] = div_by(dotp, rq.x, rq.y);
+      const bool tough = thr[u] < 0;
+      const int b = (kb & 31) + u * G + c;
+      bool fs = !tough && ((word >> b) & 1u);
+      if (hi_abs(S[u]) >= (thr[u] & 0x7fffffff)) {
+        S[u] = dotp / rq.x;
+        if (!tough && P.irrev && !fs && kb + u * G + c < len &&
+            dGT(fabs(S[u]), P.fsc * (P.rbar / sqrt(sqrt(rq.x))))) {
+          fs = true;
+          cut |= 1u << b;
+        }
+      }
+      if (kb + u * G + c < len) add |= (fs ? (P.contact ? 2u : 0u) : 1u) << (2 * u);
+    }
+    int hx = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      x[u] = m[u].x * S[u] * S[u];
+      ex[u] = exp_small(x[u]);
+      hx = max(hx, hi_abs(x[u]));
+    }
+    if (hx >= kExpSmall) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (hi_abs(x[u]) >= kExpSmall) ex[u] = exp(x[u]);
+    }
+    double p[U][3];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      double t = k4[u] * S[u] * P.C * P.beta;
+      if (thr[u] >= 0) t = t * ex[u];
+      const double s = div_by(t, P.invF, inv_invF) * m[u].y;
+      p[u][0] = s * e[u].x;
+      p[u][1] = s * e[u].y;
+      if (DIM == 3) p[u][2] = s * z[u].y;
+      if (add >> (2 * u) & 2u) {
+        double xi[3], xj[3], y[3];
+        ld_node<DIM>(D.pos64, i, xi);
+        ld_node<DIM>(D.pos64, jj[u], xj);
+        const double sf = contact64(P, xi, ui, xj, uj[u], D.vol64[i], m[u].y, y);
+        for (int q = 0; q < DIM; q++) p[u][q] = 0. + -sf * y[q];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const uint32_t a = G == 1 ? add : __shfl_sync(team, add, g, G);
+        double q[DIM];
+#pragma unroll
+        for (int h = 0; h < DIM; h++)
+          q[h] = G == 1 ? p[u][h] : __shfl_sync(team, p[u][h], g, G);
+        if (a >> (2 * u) & 3u)
+#pragma unroll
+          for (int h = 0; h < DIM; h++) fi[h] = fi[h] + q[h];
+      }
+    if (G > 1)
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) cut |= __shfl_xor_sync(team, cut, o, G);
+    if (cut) {
+      word |= cut;
+      if (c == 0) D.bits[(int64_t)(kb >> 5) * P.npad + i] = word;
+    }
+  }
+  if (c == 0) integrate_node64<DIM, SCHEME, FIRST>(P, D, T, A, i, D.flags[i], ui, fi);
+}
+
+// Teams pay the row-order additions G times but fill the chip where one thread
+// per node leaves it idle.  us per step with G = 1 / 2 / 4 / 16 -- RNPBond
+// plates of 1,600 nodes: 40 / 26 / 18 / 14, 10,000: 40 / 31 / 32 / 52, 22,500:
+// 51 / 46 / 61 / 107, 40,000: 82 / 83 / 108 / 184, 360,000: 995 / 1084 / 1267 /
+// 2287; ElasticState cubes of 1,728: 306 / 184 / 111 / 81, 8,000: 292 / 186 /
+// 173 / 248, 24,273: 431 / 371 / 414 / 683, 46,656: 688 / 737 / 814 / 1288.
+int team64(int64_t n) { return n >= 32768 ? 1 : n >= 12288 ? 2 : n >= 3072 ? 4 : 16; }
+
+cudaError_t launch_rnp_store64(const StepParams &P, const DevPtrs &D, cudaStream_t s) {
+  if (P.n == 0) return cudaSuccess;
+  auto rw = [](const double2 *p) { return const_cast<double2 *>(p); };
+  const unsigned g = (unsigned)((P.n + 127) / 128);
+  (P.dim == 2 ? k_rnp64_store<2> : k_rnp64_store<3>)<<<g, 128, 0, s>>>(
+      P, D, rw(D.b64_d), rw(D.b64_e), rw(D.b64_z), rw(D.b64_q), rw(D.b64_m),
+      const_cast<double *>(D.b64_k), const_cast<int *>(D.b64_thr));
+  return cudaGetLastError();
+}
+
 template <int DIM, int SCHEME>
 static cudaError_t launch_dim(const StepParams &P, const DevPtrs &D, const BCTable &T,
                               const StepArgs &a, cudaStream_t s) {
   const int bs = 128;
   const unsigned grid = (unsigned)((P.n + bs - 1) / bs);
   if (P.n == 0) return cudaSuccess;
-  if (a.first)
+  if (D.b64_d) {
+    const double inv = 1. / P.invF;
+    const int G = team64(P.n);
+    const unsigned gg = (unsigned)((P.n * G + kTeamBlock - 1) / kTeamBlock);
+    auto pick = [&](auto first) {
+      constexpr bool F = decltype(first)::value;
+      return G == 1   ? k_rnp64_bond<DIM, SCHEME, F, 1>
+             : G == 2 ? k_rnp64_bond<DIM, SCHEME, F, 2>
+             : G == 4 ? k_rnp64_bond<DIM, SCHEME, F, 4>
+                      : k_rnp64_bond<DIM, SCHEME, F, 16>;
+    };
+    auto kern = a.first ? pick(std::true_type{}) : pick(std::false_type{});
+    kern<<<gg, kTeamBlock, 0, s>>>(P, inv, D, T, a);
+  } else if (a.first)
     k_rnp64_thread<DIM, SCHEME, true><<<grid, bs, 0, s>>>(P, D, T, a);
   else
     k_rnp64_thread<DIM, SCHEME, false><<<grid, bs, 0, s>>>(P, D, T, a);
@@ -116,7 +338,7 @@ static cudaError_t launch_dim(const StepParams &P, const DevPtrs &D, const BCTab
 
 cudaError_t launch_rnp_step_fp64(const StepParams &P, const DevPtrs &D, const BCTable &T,
                                  const StepArgs &a, int decomp, cudaStream_t s) {
-  (void)decomp;  // the FP64 path keeps the reference summation order
+  (void)decomp;  // every FP64 path keeps the reference summation order
   if (P.dim == 2)
     return P.scheme == NLM_VELOCITY_VERLET ? launch_dim<2, NLM_VELOCITY_VERLET>(P, D, T, a, s)
                                            : launch_dim<2, NLM_CENTRAL_DIFFERENCE>(P, D, T, a, s);

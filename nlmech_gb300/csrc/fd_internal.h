@@ -35,6 +35,22 @@ struct DevPtrs {
   float4 *v32[2];  // FP32C velocity as a (hi, lo) FP32 pair, shape of u32
   double *f64;     // FP64 force density, S per node
   float *f32;      // FP32C force density, S per node
+  // FP64 bond store: what a step needs of a bond's reference geometry, in the
+  // sliced-ELL shape with entry k of lane l at sell_ptr + 32 k + l (null: the
+  // step kernels recompute it, see build_bond_store64)
+  const double2 *b64_d;   // RNPBond: reference bond vector (x, y)
+  const double2 *b64_e;   // its direction (x, y)
+  const double2 *b64_z;   // 3-D: z of the vector and of the direction
+  const double2 *b64_q;   // |xi|^2 and its reciprocal
+  const double2 *b64_m;   // -beta |xi| and the corrected volume of j
+  const double *b64_k;    // 4 J(|xi| / delta); null when J is constant
+  const int *b64_thr;     // high word of the break threshold (see fd_fp64.cu)
+  const double2 *es64_x;  // ElasticState: |X| and the volume factor omega
+  const double *es64_v;   // V_j
+  const int *es64_thr;    // high word of a lower bound of the extension at s_c
+  double *es64_yl;        // |Y| of the current step, pass 1 to pass 2
+  const double2 *es64_c;  // per node: coefficients of e_s and e_d
+  double *es64_y;         // per node: x + u of the current step, S doubles
   // ElasticState
   const double *mw64;     // weighted volume m_i
   const float *minv32;    // FP32C: 1 / m_i formed in FP64, rounded once
@@ -103,6 +119,12 @@ cudaError_t launch_es_step_fp64(const StepParams &P, const DevPtrs &D, const BCT
                                 const StepArgs &a, int decomp, cudaStream_t s);
 cudaError_t launch_es_step_fp32(const StepParams &P, const DevPtrs &D, const BCTable &T,
                                 const StepArgs &a, int decomp, cudaStream_t s);
+// Lanes per node of the FP64 bond-store kernels, and their block size.
+int team64(int64_t n);
+constexpr int kTeamBlock = 64;
+// Fill the FP64 bond stores (arrays of D allocated by the caller).
+cudaError_t launch_rnp_store64(const StepParams &P, const DevPtrs &D, cudaStream_t s);
+cudaError_t launch_es_store64(const StepParams &P, const DevPtrs &D, cudaStream_t s);
 // Recompute the drift to u^{m+1} (and v^{m+1} for CD) from (u^m, v^m, f^m)
 // after the host replaced the state: the second half of the step epilogue.
 cudaError_t launch_drift(const StepParams &P, const DevPtrs &D, const BCTable &T, int cur,

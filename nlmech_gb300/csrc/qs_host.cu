@@ -127,7 +127,7 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
   d.decomposition = NLM_DECOMP_THREAD;
   if (!(d.dt > 0.)) return fail(NLM_ERR_INVALID, "load-step increment dt must be positive");
   nlm_qs *q = new nlm_qs();
-  int rc = nlm_fd_create(&d, &q->fd);
+  int rc = create_model(&d, &q->fd, false);
   if (rc) {
     delete q;
     return rc;

@@ -17,6 +17,9 @@ struct nlm_esqs {
   double *theta = nullptr, *f = nullptr, *body = nullptr, *res = nullptr, *rhs = nullptr;
   double *dx = nullptr, *J = nullptr, *r = nullptr, *rhat = nullptr, *p = nullptr;
   double *v = nullptr, *sv = nullptr, *t = nullptr, *part = nullptr, *sc = nullptr;
+  // Jacobian assembly: per-bond differences, row and original column of a bond
+  double *bond = nullptr;
+  int *rows = nullptr, *ocols = nullptr;
   std::vector<void *> allocs;
   ~nlm_esqs() {
     if (fd) nlm_fd_destroy(fd);  // synchronises and frees the stream first
@@ -171,7 +174,12 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   for (double **ptr : {&q->f, &q->body, &q->res, &q->rhs, &q->dx, &q->r, &q->rhat, &q->p, &q->v,
                        &q->sv, &q->t})
     if (e == cudaSuccess) e = q->alloc(ptr, q->m);
-  if (e == cudaSuccess) e = q->alloc(&q->J, (size_t)9 * q->nblocks);
+  const size_t md = (size_t)q->mdim;
+  if (e == cudaSuccess) e = q->alloc(&q->J, md * md * q->nblocks);
+  if (e == cudaSuccess) e = q->alloc(&q->bond, (3 * md + md * md) * (size_t)h->nnz);
+  if (e == cudaSuccess) e = q->alloc(&q->rows, (size_t)h->nnz);
+  if (e == cudaSuccess) e = q->alloc(&q->ocols, (size_t)h->nnz);
+  if (e == cudaSuccess) e = esqs_topology(h->P, h->D, q->rows, q->ocols, h->stream);
   if (e == cudaSuccess) e = q->alloc(&q->part, kEsqsDotParts);
   if (e == cudaSuccess) e = q->alloc(&q->sc, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(q->body, 0, sizeof(double) * q->m, h->stream);
@@ -217,8 +225,9 @@ int nlm_esqs_solve(nlm_esqs *q, int nsteps, int *newton_iters, int *lin_iters,
       return q->prm.tol_relative ? (r0 == 0. || res / r0 < q->prm.tol) : res < q->prm.tol;
     };
     while (!converged() && it < q->prm.max_iters) {
-      cudaError_t e = esqs_jacobian(h->P, h->D, h->S, q->mdim, q->prm.jacobian, u, eps, q->J,
-                                    q->nblocks, s);
+      // theta is esqs_eval's, at the current u
+      cudaError_t e = esqs_jacobian(h->P, h->D, h->S, q->mdim, q->prm.jacobian, u, q->theta, eps,
+                                    h->nnz, q->rows, q->ocols, q->bond, q->J, s);
       if (e == cudaSuccess) e = esqs_lin3(q->m, -1., q->res, 0., nullptr, 0., nullptr, q->rhs, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static Jacobian");
       int li = 0;

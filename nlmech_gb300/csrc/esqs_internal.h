@@ -16,9 +16,14 @@ cudaError_t esqs_force(const StepParams &P, const DevPtrs &D, int S, int mdim, c
 // r = f + b on free dofs, 0 on fixed dofs.
 cudaError_t esqs_residual(const StepParams &P, const DevPtrs &D, int S, int mdim,
                           const double *f, const double *b, double *r, cudaStream_t s);
-// Finite-difference Jacobian blocks (9 doubles each, nblocks = nnz + n).
+// rows, ocols: row node and original column id of every directed bond
+cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *rows, int *ocols,
+                          cudaStream_t s);
+// Jacobian blocks (mdim^2 each, nnz + n of them) at u; theta: the dilatations
+// at u; bond: 3 mdim + mdim^2 doubles per directed bond
 cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim, int full,
-                          const double *u, double eps, double *J, int64_t nblocks,
+                          const double *u, const double *theta, double eps, int64_t nnz,
+                          const int *rows, const int *ocols, double *bond, double *J,
                           cudaStream_t s);
 cudaError_t esqs_spmv(const StepParams &P, const DevPtrs &D, int S, int mdim, const double *J,
                       const double *x, double *y, cudaStream_t s);

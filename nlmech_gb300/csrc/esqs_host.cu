@@ -15,8 +15,8 @@ struct nlm_esqs {
   int mdim = 2;
   int64_t m = 0, nblocks = 0;
   double *theta = nullptr, *f = nullptr, *body = nullptr, *res = nullptr, *rhs = nullptr;
-  double *dx = nullptr, *J = nullptr, *r = nullptr, *rhat = nullptr, *p = nullptr;
-  double *v = nullptr, *sv = nullptr, *t = nullptr, *part = nullptr, *sc = nullptr;
+  double *dx = nullptr, *J = nullptr, *part = nullptr, *sc = nullptr;
+  BiArgs bi{};
   // Jacobian assembly: per-bond differences, row and original column of a bond
   double *bond = nullptr;
   int *rows = nullptr, *ocols = nullptr;
@@ -57,72 +57,6 @@ int esqs_eval(nlm_esqs *q, double *norm) {
   int rc = esqs_dot_host(q, q->res, q->res, &rr);
   *norm = std::sqrt(rr);
   return rc;
-}
-
-// BiCGSTAB (van der Vorst 1992) for J dx = rhs to ||r|| <= tol ||rhs||.
-int esqs_bicgstab(nlm_esqs *q, int *iters) {
-  nlm_fd *h = q->fd;
-  cudaStream_t s = h->stream;
-  const int64_t m = q->m;
-  const size_t bytes = sizeof(double) * m;
-  NLM_CUDA(cudaMemsetAsync(q->dx, 0, bytes, s));
-  NLM_CUDA(cudaMemcpyAsync(q->r, q->rhs, bytes, cudaMemcpyDeviceToDevice, s));
-  NLM_CUDA(cudaMemcpyAsync(q->rhat, q->rhs, bytes, cudaMemcpyDeviceToDevice, s));
-  NLM_CUDA(cudaMemsetAsync(q->p, 0, bytes, s));
-  NLM_CUDA(cudaMemsetAsync(q->v, 0, bytes, s));
-  double bb = 0.;
-  int rc = esqs_dot_host(q, q->rhs, q->rhs, &bb);
-  if (rc) return rc;
-  *iters = 0;
-  const double bnorm = std::sqrt(bb);
-  if (bnorm == 0.) return NLM_OK;
-  const double stop = q->prm.lin_tol * bnorm;
-  double rho = 1., alpha = 1., omega = 1.;
-  auto J_times = [&](const double *x, double *y) {
-    cudaError_t e = esqs_spmv(h->P, h->D, h->S, q->mdim, q->J, x, y, s);
-    return e == cudaSuccess ? NLM_OK : cuda_fail(e, "quasi-static Jacobian product");
-  };
-  auto lin3 = [&](double a, const double *x, double b, const double *y, double c, const double *z,
-                  double *out) {
-    cudaError_t e = esqs_lin3(m, a, x, b, y, c, z, out, s);
-    return e == cudaSuccess ? NLM_OK : cuda_fail(e, "quasi-static vector update");
-  };
-  for (int it = 1; it <= q->prm.lin_max_iters; it++) {
-    *iters = it;
-    double rho_new = 0.;
-    if ((rc = esqs_dot_host(q, q->rhat, q->r, &rho_new))) return rc;
-    if (rho_new == 0.) break;  // breakdown: keep the iterate
-    const double beta = (rho_new / rho) * (alpha / omega);
-    if ((rc = lin3(1., q->r, beta, q->p, -beta * omega, q->v, q->p))) return rc;
-    if ((rc = J_times(q->p, q->v))) return rc;
-    double rv = 0.;
-    if ((rc = esqs_dot_host(q, q->rhat, q->v, &rv))) return rc;
-    if (rv == 0.) break;
-    alpha = rho_new / rv;
-    if ((rc = lin3(1., q->r, -alpha, q->v, 0., nullptr, q->sv))) return rc;
-    double ss = 0.;
-    if ((rc = esqs_dot_host(q, q->sv, q->sv, &ss))) return rc;
-    if (std::sqrt(ss) <= stop) {
-      if ((rc = lin3(1., q->dx, alpha, q->p, 0., nullptr, q->dx))) return rc;
-      break;
-    }
-    if ((rc = J_times(q->sv, q->t))) return rc;
-    double ts = 0., tt = 0.;
-    if ((rc = esqs_dot_host(q, q->t, q->sv, &ts))) return rc;
-    if ((rc = esqs_dot_host(q, q->t, q->t, &tt))) return rc;
-    if (tt == 0.) {
-      if ((rc = lin3(1., q->dx, alpha, q->p, 0., nullptr, q->dx))) return rc;
-      break;
-    }
-    omega = ts / tt;
-    if ((rc = lin3(1., q->dx, alpha, q->p, omega, q->sv, q->dx))) return rc;
-    if ((rc = lin3(1., q->sv, -omega, q->t, 0., nullptr, q->r))) return rc;
-    double rr = 0.;
-    if ((rc = esqs_dot_host(q, q->r, q->r, &rr))) return rc;
-    if (std::sqrt(rr) <= stop || omega == 0.) break;
-    rho = rho_new;
-  }
-  return NLM_OK;
 }
 
 }  // namespace
@@ -171,9 +105,14 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   q->m = (int64_t)h->S * h->n;
   q->nblocks = h->nnz + h->n;
   cudaError_t e = q->alloc(&q->theta, h->n);
-  for (double **ptr : {&q->f, &q->body, &q->res, &q->rhs, &q->dx, &q->r, &q->rhat, &q->p, &q->v,
-                       &q->sv, &q->t})
+  BiArgs &bi = q->bi;
+  for (double **ptr : {&q->f, &q->body, &q->res, &q->rhs, &q->dx, &bi.r, &bi.rhat, &bi.p[0],
+                       &bi.p[1], &bi.v[0], &bi.v[1], &bi.s, &bi.t})
     if (e == cudaSuccess) e = q->alloc(ptr, q->m);
+  if (e == cudaSuccess) e = q->alloc(&bi.part1, kBiParts);
+  if (e == cudaSuccess) e = q->alloc(&bi.part2, 3 * kBiParts);
+  if (e == cudaSuccess) e = q->alloc(&bi.part3, 2 * kBiParts);
+  if (e == cudaSuccess) e = q->alloc(&bi.sc, 6);
   const size_t md = (size_t)q->mdim;
   if (e == cudaSuccess) e = q->alloc(&q->J, md * md * q->nblocks);
   if (e == cudaSuccess) e = q->alloc(&q->bond, (3 * md + md * md) * (size_t)h->nnz);
@@ -182,6 +121,14 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   if (e == cudaSuccess) e = esqs_topology(h->P, h->D, q->rows, q->ocols, h->stream);
   if (e == cudaSuccess) e = q->alloc(&q->part, kEsqsDotParts);
   if (e == cudaSuccess) e = q->alloc(&q->sc, 1);
+  bi.n = h->n;
+  bi.m = q->m;
+  bi.flags = h->D.flags;
+  bi.rowptr = h->D.rowptr;
+  bi.cols = h->D.cols;
+  bi.J = q->J;
+  bi.x = q->dx;
+  esqs_bicgstab_grid(h->n, q->m, bi);
   if (e == cudaSuccess) e = cudaMemsetAsync(q->body, 0, sizeof(double) * q->m, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
@@ -231,7 +178,8 @@ int nlm_esqs_solve(nlm_esqs *q, int nsteps, int *newton_iters, int *lin_iters,
       if (e == cudaSuccess) e = esqs_lin3(q->m, -1., q->res, 0., nullptr, 0., nullptr, q->rhs, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static Jacobian");
       int li = 0;
-      if ((rc = esqs_bicgstab(q, &li))) return rc;
+      e = esqs_bicgstab(q->bi, q->mdim, q->rhs, q->prm.lin_tol, q->prm.lin_max_iters, &li, s);
+      if (e != cudaSuccess) return cuda_fail(e, "quasi-static linear solve");
       li_total += li;
       e = esqs_lin3(q->m, 1., u, 1., q->dx, 0., nullptr, u, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static update");

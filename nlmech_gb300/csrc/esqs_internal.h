@@ -25,8 +25,28 @@ cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim
                           const double *u, const double *theta, double eps, int64_t nnz,
                           const int *rows, const int *ocols, double *bond, double *J,
                           cudaStream_t s);
-cudaError_t esqs_spmv(const StepParams &P, const DevPtrs &D, int S, int mdim, const double *J,
-                      const double *x, double *y, cudaStream_t s);
+// BiCGSTAB state on the device (sc: two slots, by iteration parity, for each of
+// the three launches of an iteration).
+struct BiScal {
+  double rho, alpha, omega, stop;
+  int done, iters;
+};
+constexpr int kBiParts = 512;  // most blocks of a launch
+struct BiArgs {
+  int64_t n, m;             // nodes, entries of a vector (S per node)
+  const uint8_t *flags;
+  const int64_t *rowptr;
+  const int *cols;
+  const double *J;
+  double *r, *rhat, *p[2], *v[2], *s, *t, *x;
+  double *part1, *part2, *part3;  // kBiParts, 3 and 2 times kBiParts doubles
+  int np1, np3;                   // blocks of the product and update launches
+  BiScal *sc;                     // 6
+};
+void esqs_bicgstab_grid(int64_t n, int64_t m, BiArgs &B);
+// J x = rhs to ||r|| <= tol ||rhs||, at most max_iters iterations; synchronises.
+cudaError_t esqs_bicgstab(const BiArgs &B, int mdim, const double *rhs, double tol, int max_iters,
+                          int *iters, cudaStream_t s);
 // out = a x + b y + c z; y or z may be NULL.
 cudaError_t esqs_lin3(int64_t m, double a, const double *x, double b, const double *y, double c,
                       const double *z, double *out, cudaStream_t s);

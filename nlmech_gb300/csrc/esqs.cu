@@ -371,29 +371,30 @@ __device__ __forceinline__ void bi_row(const BiArgs &B, int64_t i, int g, V val,
 }
 
 template <int MD>
-__global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k, double tol) {
+__global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k) {
   constexpr int S = MD == 3 ? 4 : 2;
   pdl_trigger_and_wait();
-  const BiScal in = B.sc[4 + ((k - 1) & 1)];
+  const BiScal in = B.sc[4 + ((k ^ 1) & 1)];
   BiScal out = in;
   double tot[2];
   if (!in.done) {
     bi_totals<2>(B.part3, B.np3, tot);
     const double rnorm = sqrt(tot[1]);
-    if (k == 1) out.stop = tol * rnorm;
-    if (k == 1 ? rnorm == 0. : (rnorm <= in.stop || in.omega == 0.)) {
+    const bool first = in.iters == 0;
+    if (first) out.stop = B.tol * rnorm;
+    if ((first ? rnorm == 0. : (rnorm <= in.stop || in.omega == 0.)) ||
+        in.iters >= B.max_iters) {
       out.done = 1;
-      out.iters = k - 1;
     } else {
       out.done = tot[0] == 0.;  // breakdown: keep the iterate
-      out.iters = k;
+      out.iters = in.iters + 1;
       out.rho = tot[0];
     }
   }
   bi_store(B.sc + (k & 1), out);
   if (out.done) return;
   const double beta = (tot[0] / in.rho) * (in.alpha / in.omega), bo = -beta * in.omega;
-  const double *po = B.p[(k - 1) & 1], *vo = B.v[(k - 1) & 1];
+  const double *po = B.p[(k ^ 1) & 1], *vo = B.v[(k ^ 1) & 1];
   double *pn = B.p[k & 1], *vn = B.v[k & 1];
   const int g = threadIdx.x % kBiTeam;
   double rv[1] = {};
@@ -594,31 +595,38 @@ void esqs_bicgstab_grid(int64_t n, int64_t m, BiArgs &B) {
                                  std::min<int64_t>(kBiParts, (m + kBiThreads - 1) / kBiThreads));
 }
 
-cudaError_t esqs_bicgstab(const BiArgs &B, int mdim, const double *rhs, double tol, int max_iters,
-                          int *iters, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  k_bi_init<<<B.np3, kBiThreads, 0, s>>>(B, rhs);
-  BiScal st{};
-  *iters = max_iters;
+// kBiGraph iterations as one CUDA graph (iteration parities 1, 0, 1, ...).
+cudaError_t esqs_bicgstab_graph(const BiArgs &B, int mdim, cudaGraphExec_t *out, cudaStream_t s) {
   auto dir = mdim == 1 ? k_bi_dir<1> : mdim == 2 ? k_bi_dir<2> : k_bi_dir<3>;
   auto shadow = mdim == 1 ? k_bi_shadow<1> : mdim == 2 ? k_bi_shadow<2> : k_bi_shadow<3>;
-  for (int k = 1; k <= max_iters;) {
-    // a look at the state costs about as much as two iterations
-    const int end = std::min(max_iters, k + 31);
-    for (; k <= end && e == cudaSuccess; k++) {
-      e = launch_pdl(dir, B.np1, kBiThreads, 0, s, k > 1, B, k, tol);
-      if (e == cudaSuccess) e = launch_pdl(shadow, B.np1, kBiThreads, 0, s, true, B, k);
-      if (e == cudaSuccess) e = launch_pdl(k_bi_update, B.np3, kBiThreads, 0, s, true, B, k);
-    }
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&st, B.sc + ((k - 1) & 1), sizeof(st), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    if (st.done) {
-      *iters = st.iters;
-      break;
-    }
+  cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  for (int k = 1; k <= kBiGraph && e == cudaSuccess; k++) {
+    e = launch_pdl(dir, B.np1, kBiThreads, 0, s, k > 1, B, k & 1);
+    if (e == cudaSuccess) e = launch_pdl(shadow, B.np1, kBiThreads, 0, s, true, B, k & 1);
+    if (e == cudaSuccess) e = launch_pdl(k_bi_update, B.np3, kBiThreads, 0, s, true, B, k & 1);
   }
+  cudaGraph_t g = nullptr;
+  const cudaError_t ec = cudaStreamEndCapture(s, &g);
+  if (e == cudaSuccess) e = ec;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+  if (g) cudaGraphDestroy(g);
+  return e;
+}
+
+cudaError_t esqs_bicgstab(const BiArgs &B, cudaGraphExec_t graph, const double *rhs, int *iters,
+                          cudaStream_t s) {
+  k_bi_init<<<B.np3, kBiThreads, 0, s>>>(B, rhs);
+  cudaError_t e = cudaGetLastError();
+  BiScal st{};
+  // the state after each graph's last direction launch; max_iters ends the loop
+  while (e == cudaSuccess && !st.done && st.iters < B.max_iters) {
+    e = cudaGraphLaunch(graph, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&st, B.sc + 4, sizeof(st), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
+  *iters = st.iters;
   return e;
 }
 

@@ -17,11 +17,14 @@ struct nlm_esqs {
   double *theta = nullptr, *f = nullptr, *body = nullptr, *res = nullptr, *rhs = nullptr;
   double *dx = nullptr, *J = nullptr, *part = nullptr, *sc = nullptr;
   BiArgs bi{};
+  cudaGraphExec_t bi_graph = nullptr;
   // Jacobian assembly: per-bond differences, row and original column of a bond
   double *bond = nullptr;
   int *rows = nullptr, *ocols = nullptr;
   std::vector<void *> allocs;
   ~nlm_esqs() {
+    if (fd && fd->stream) cudaStreamSynchronize(fd->stream);
+    if (bi_graph) cudaGraphExecDestroy(bi_graph);
     if (fd) nlm_fd_destroy(fd);  // synchronises and frees the stream first
     for (void *q : allocs) cudaFree(q);
   }
@@ -128,6 +131,8 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   bi.cols = h->D.cols;
   bi.J = q->J;
   bi.x = q->dx;
+  bi.tol = prm->lin_tol;
+  bi.max_iters = prm->lin_max_iters;
   esqs_bicgstab_grid(h->n, q->m, bi);
   if (e == cudaSuccess) e = cudaMemsetAsync(q->body, 0, sizeof(double) * q->m, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -178,7 +183,8 @@ int nlm_esqs_solve(nlm_esqs *q, int nsteps, int *newton_iters, int *lin_iters,
       if (e == cudaSuccess) e = esqs_lin3(q->m, -1., q->res, 0., nullptr, 0., nullptr, q->rhs, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static Jacobian");
       int li = 0;
-      e = esqs_bicgstab(q->bi, q->mdim, q->rhs, q->prm.lin_tol, q->prm.lin_max_iters, &li, s);
+      if (!q->bi_graph) e = esqs_bicgstab_graph(q->bi, q->mdim, &q->bi_graph, s);
+      if (e == cudaSuccess) e = esqs_bicgstab(q->bi, q->bi_graph, q->rhs, &li, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static linear solve");
       li_total += li;
       e = esqs_lin3(q->m, 1., u, 1., q->dx, 0., nullptr, u, s);

@@ -42,11 +42,15 @@ struct BiArgs {
   double *part1, *part2, *part3;  // kBiParts, 3 and 2 times kBiParts doubles
   int np1, np3;                   // blocks of the product and update launches
   BiScal *sc;                     // 6
+  double tol;                     // ||r|| <= tol ||rhs||
+  int max_iters;
 };
+constexpr int kBiGraph = 32;  // iterations per graph launch (even)
 void esqs_bicgstab_grid(int64_t n, int64_t m, BiArgs &B);
-// J x = rhs to ||r|| <= tol ||rhs||, at most max_iters iterations; synchronises.
-cudaError_t esqs_bicgstab(const BiArgs &B, int mdim, const double *rhs, double tol, int max_iters,
-                          int *iters, cudaStream_t s);
+cudaError_t esqs_bicgstab_graph(const BiArgs &B, int mdim, cudaGraphExec_t *out, cudaStream_t s);
+// J x = rhs; synchronises.
+cudaError_t esqs_bicgstab(const BiArgs &B, cudaGraphExec_t graph, const double *rhs, int *iters,
+                          cudaStream_t s);
 // out = a x + b y + c z; y or z may be NULL.
 cudaError_t esqs_lin3(int64_t m, double a, const double *x, double b, const double *y, double c,
                       const double *z, double *out, cudaStream_t s);

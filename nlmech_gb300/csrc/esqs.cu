@@ -277,139 +277,194 @@ __global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *rows, int *ocol
 }
 
 // ---- BiCGSTAB (van der Vorst 1992) --------------------------------------------
-// One iteration is three launches with every scalar on the device:
-//   dir:    beta, p = r + beta (p - omega v), v = J p, partials of rhat.v
-//   shadow: alpha, s = r - alpha v, t = J s, partials of s.s, t.s, t.t
-//   update: omega, x += alpha p + omega s, r = s - omega t, partials of
-//           rhat.r and r.r
+// One iteration is two launches with every scalar on the device:
+//   dir:    ends the last iteration -- omega, x += alpha p + omega s, r = s -
+//           omega t -- and starts the next: beta, p = r + beta (p - omega v),
+//           v = J p, partials of rhat.v
+//   shadow: alpha, s = r - alpha v, t = J s, partials of s.s, t.s, t.t, rhat.s
+//           and rhat.t
+// r.r and rhat.r follow from shadow's sums (r = s - omega t with omega =
+// t.s / t.t), which saves the third launch a separate sum over r would need.  r,
 // p and s of a neighbour are formed where the product reads them, partial sums
-// are added by every block of the next launch in one fixed order, and a launch
-// after convergence does nothing, so the host looks at the state once in many
-// iterations.  It used to wait for the GPU six times per iteration: a load step
-// of the 40 x 36 plate (418 iterations) took 89 ms, now 13.9 ms.  What bounds it
-// is the latency of three dependent launches per iteration.
+// are added by one warp of every block of the next launch in one fixed order
+// while the others fetch their blocks of J, and a launch after convergence does
+// nothing, so the host looks at the state once per graph of kBiGraph
+// iterations.  A load step of the 40 x 36 plate (418 iterations): 89 ms with six
+// host waits per iteration, 13.4 ms with three launches (blocks of 128, every
+// thread forming the totals), 12.2 ms now.  Bound: two dependent launches, and the
+// FP64 latency of the sums (2 FP64 lanes per SM), hence the small blocks.
 
-constexpr int kBiThreads = 128;
+constexpr int kBiThreads = 64;
 constexpr int kBiTeam = 8;  // lanes per row of J
 
-__device__ __forceinline__ void bi_store(BiScal *o, const BiScal &v) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *o = v;
-}
-
-// Totals of N partial arrays of np entries each, in one fixed order.
+// Totals of N partial arrays of gridDim.x entries each, in one fixed order
+// (one warp; lane 0 ends with them).
 template <int N>
-__device__ __forceinline__ void bi_totals(const double *part, int np, double tot[N]) {
-  __shared__ double sh[N][kBiThreads / 32];
-  double v[N] = {};
-  for (int k = threadIdx.x; k < np; k += kBiThreads)
-    for (int a = 0; a < N; a++) v[a] += __ldcg(part + a * np + k);
+__device__ __forceinline__ void bi_totals(const double *part, double tot[N]) {
+  const int np = (int)gridDim.x;
+  for (int a = 0; a < N; a++) tot[a] = 0.;
+  for (int k = threadIdx.x & 31; k < np; k += 32)
+#pragma unroll
+    for (int a = 0; a < N; a++) tot[a] += __ldcg(part + a * np + k);
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1)
-    for (int a = 0; a < N; a++) v[a] += __shfl_xor_sync(0xffffffffu, v[a], o);
-  if ((threadIdx.x & 31) == 0)
-    for (int a = 0; a < N; a++) sh[a][threadIdx.x >> 5] = v[a];
-  __syncthreads();
-  for (int a = 0; a < N; a++) {
-    tot[a] = 0.;
-    for (int w = 0; w < kBiThreads / 32; w++) tot[a] += sh[a][w];
-  }
-  __syncthreads();
+#pragma unroll
+    for (int a = 0; a < N; a++) tot[a] += __shfl_xor_sync(0xffffffffu, tot[a], o);
 }
 
 // Block sums of N values per thread into part[a * gridDim.x + blockIdx.x].
 template <int N>
-__device__ __forceinline__ void bi_partials(const double val[N], double *part) {
-  __shared__ double sh[N][kBiThreads / 32];
-  double v[N];
-  for (int a = 0; a < N; a++) v[a] = val[a];
+__device__ __forceinline__ void bi_partials(double v[N], double *part) {
+  static_assert(kBiThreads == 64, "two warps");
+  __shared__ double sh[N];
   for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
     for (int a = 0; a < N; a++) v[a] += __shfl_xor_sync(0xffffffffu, v[a], o);
-  if ((threadIdx.x & 31) == 0)
-    for (int a = 0; a < N; a++) sh[a][threadIdx.x >> 5] = v[a];
+  if (threadIdx.x == 32)
+    for (int a = 0; a < N; a++) sh[a] = v[a];
   __syncthreads();
   if (threadIdx.x == 0)
-    for (int a = 0; a < N; a++) {
-      double t = 0.;
-      for (int w = 0; w < kBiThreads / 32; w++) t += sh[a][w];
-      part[a * gridDim.x + blockIdx.x] = t;
-    }
+    for (int a = 0; a < N; a++) part[a * gridDim.x + blockIdx.x] = v[a] + sh[a];
 }
 
-// r = rhat = rhs, x = p = v = 0, partials of r.r (twice: rho and r.r).
+// s = r = rhat = rhs, the other vectors 0, shadow's partials for omega = 0.
 __global__ void __launch_bounds__(kBiThreads) k_bi_init(const BiArgs B, const double *rhs) {
-  double rr[2] = {};
+  double sum[5] = {};
   for (int64_t q = blockIdx.x * (int64_t)kBiThreads + threadIdx.x; q < B.m;
        q += (int64_t)gridDim.x * kBiThreads) {
     const double b = rhs[q];
-    B.r[q] = b;
-    B.rhat[q] = b;
+    B.s[q] = B.rhat[q] = b;
     // (components a row does not write stay zero)
-    B.x[q] = B.p[0][q] = B.p[1][q] = B.v[0][q] = B.v[1][q] = B.s[q] = B.t[q] = 0.;
-    rr[0] += b * b;
+    B.r[q] = B.x[q] = B.p[0][q] = B.p[1][q] = B.v[0][q] = B.v[1][q] = B.t[q] = 0.;
+    sum[0] += b * b;
   }
-  rr[1] = rr[0];
-  bi_partials<2>(rr, B.part3);
-  bi_store(B.sc + 4, BiScal{1., 1., 1., 0., 0, 0});
+  sum[3] = sum[0];
+  bi_partials<5>(sum, B.part2);
+  if (blockIdx.x == 0 && threadIdx.x == 0) B.sc[2] = BiScal{1., 0., 0., 0., 0., 0, 0};
 }
 
-// Row i of J times y, y_j given by val(j, y); the team's lanes end with the sum.
-template <int MD, class V>
-__device__ __forceinline__ void bi_row(const BiArgs &B, int64_t i, int g, V val, double acc[MD]) {
-  const int64_t r0 = B.rowptr[i];
-  const int len = (int)(B.rowptr[i + 1] - r0);
-  for (int d = 0; d < MD; d++) acc[d] = 0.;
-  for (int b = g; b <= len; b += kBiTeam) {
-    const int64_t j = b == 0 ? i : (int64_t)B.cols[r0 + b - 1];
-    const double *blk = B.J + MD * MD * (r0 + i + b);
-    double y[MD];
-    val(j, y);
-    for (int ss = 0; ss < MD; ss++)
-      for (int rr = 0; rr < MD; rr++)
-        acc[ss] = __fma_rn(blk[ss * MD + rr], y[rr], acc[ss]);
+// A team's share of row i of J (block b = g, g + 8, ...): the first PF blocks
+// are fetched ahead of the launch's scalars.
+template <int MD>
+struct BiRow {
+  static constexpr int PF = MD == 3 ? 2 : 4;
+  int64_t r0, i;
+  int len, col[PF];
+  double blk[PF][MD * MD];
+  __device__ __forceinline__ int64_t column(const BiArgs &B, int b) const {
+    return b == 0 ? i : (int64_t)B.cols[r0 + b - 1];
   }
-  for (int o = kBiTeam / 2; o > 0; o >>= 1)
-    for (int d = 0; d < MD; d++) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
-}
+  __device__ __forceinline__ void fetch(const BiArgs &B, int64_t row, int g) {
+    i = row;
+    r0 = B.rowptr[i];
+    len = (int)(B.rowptr[i + 1] - r0);
+#pragma unroll
+    for (int u = 0; u < PF; u++) {
+      const int b = g + u * kBiTeam;
+      col[u] = b <= len ? (int)column(B, b) : -1;
+#pragma unroll
+      for (int d = 0; d < MD * MD; d++)
+        blk[u][d] = b <= len ? __ldg(B.J + MD * MD * (r0 + i + b) + d) : 0.;
+    }
+  }
+  // acc = J_i y with y_j from val(j, y), the same in all lanes of the team
+  template <class V>
+  __device__ __forceinline__ void times(const BiArgs &B, int g, V val, double acc[MD]) const {
+    for (int d = 0; d < MD; d++) acc[d] = 0.;
+    auto add = [&](int64_t j, const double *a) {
+      double y[MD];
+      val(j, y);
+      for (int ss = 0; ss < MD; ss++)
+        for (int rr = 0; rr < MD; rr++) acc[ss] = __fma_rn(a[ss * MD + rr], y[rr], acc[ss]);
+    };
+#pragma unroll
+    for (int u = 0; u < PF; u++)
+      if (col[u] >= 0) add(col[u], blk[u]);
+    for (int b = g + PF * kBiTeam; b <= len; b += kBiTeam) {
+      double a[MD * MD];
+      for (int d = 0; d < MD * MD; d++) a[d] = __ldg(B.J + MD * MD * (r0 + i + b) + d);
+      add(column(B, b), a);
+    }
+    for (int o = kBiTeam / 2; o > 0; o >>= 1)
+      for (int d = 0; d < MD; d++) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
+  }
+};
+
+constexpr int64_t kBiRows = kBiThreads / kBiTeam;  // rows of a block
 
 template <int MD>
 __global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k) {
   constexpr int S = MD == 3 ? 4 : 2;
-  pdl_trigger_and_wait();
-  const BiScal in = B.sc[4 + ((k ^ 1) & 1)];
-  BiScal out = in;
-  double tot[2];
-  if (!in.done) {
-    bi_totals<2>(B.part3, B.np3, tot);
-    const double rnorm = sqrt(tot[1]);
-    const bool first = in.iters == 0;
-    if (first) out.stop = B.tol * rnorm;
-    if ((first ? rnorm == 0. : (rnorm <= in.stop || in.omega == 0.)) ||
-        in.iters >= B.max_iters) {
-      out.done = 1;
-    } else {
-      out.done = tot[0] == 0.;  // breakdown: keep the iterate
-      out.iters = in.iters + 1;
-      out.rho = tot[0];
+  __shared__ BiScal s_sc;
+  const int g = threadIdx.x % kBiTeam;
+  const int64_t first_row = blockIdx.x * kBiRows + threadIdx.x / kBiTeam;
+  BiRow<MD> row;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  row.fetch(B, min(first_row, B.n - 1), g);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (threadIdx.x < 32) {
+    BiScal sc = B.sc[2 + ((k ^ 1) & 1)];
+    double t[5];  // s.s, t.s, t.t, rhat.s, rhat.t
+    bi_totals<5>(B.part2, t);
+    if (threadIdx.x == 0) {
+      if (!sc.done) {
+        const double rho = sc.rho;
+        if (sc.iters == 0) {
+          sc.stop2 = B.tol * B.tol * t[0];
+          sc.rho = t[3];
+          sc.beta = sc.omega = 0.;
+          sc.done = t[0] == 0.;
+        } else {
+          const bool half = t[0] <= sc.stop2 || t[2] == 0.;
+          sc.omega = half ? 0. : t[1] / t[2];
+          sc.rho = __fma_rn(-sc.omega, t[4], t[3]);
+          sc.beta = (sc.rho / rho) * (sc.alpha / sc.omega);
+          sc.done = half || __fma_rn(-sc.omega, t[1], t[0]) <= sc.stop2 || sc.omega == 0. ||
+                    sc.iters >= B.max_iters;
+        }
+        if (!sc.done) {
+          sc.iters++;
+          if (sc.rho == 0.) sc.done = 1;  // breakdown: keep the iterate
+        }
+        // the solve's last x update is still due in this launch
+        sc.done = sc.done ? 2 : 0;
+      } else {
+        sc.done = 1;
+      }
+      s_sc = sc;
+      if (blockIdx.x == 0) B.sc[k & 1] = sc;
     }
   }
-  bi_store(B.sc + (k & 1), out);
-  if (out.done) return;
-  const double beta = (tot[0] / in.rho) * (in.alpha / in.omega), bo = -beta * in.omega;
+  __syncthreads();
+  const BiScal sc = s_sc;
+  if (sc.done == 1) return;
   const double *po = B.p[(k ^ 1) & 1], *vo = B.v[(k ^ 1) & 1];
   double *pn = B.p[k & 1], *vn = B.v[k & 1];
-  const int g = threadIdx.x % kBiTeam;
+  const double bo = -sc.beta * sc.omega;
   double rv[1] = {};
-  constexpr int64_t R = kBiThreads / kBiTeam;
-  for (int64_t i0 = blockIdx.x * R; i0 < B.n; i0 += gridDim.x * R) {
-    const int64_t it = i0 + threadIdx.x / kBiTeam, i = it < B.n ? it : B.n - 1;
+  for (int64_t i0 = blockIdx.x * kBiRows; i0 < B.n; i0 += gridDim.x * kBiRows) {
+    const int64_t it = i0 + threadIdx.x / kBiTeam;
+    if (it != first_row) row.fetch(B, min(it, B.n - 1), g);
+    const int64_t i = row.i;
+    const bool own = g == 0 && it < B.n;
+    if (own)
+      for (int d = 0; d < MD; d++) {
+        const int64_t q = S * i + d;
+        const double s = B.s[q];
+        B.x[q] = __fma_rn(sc.omega, s, __fma_rn(sc.alpha, po[q], B.x[q]));
+        B.r[q] = __fma_rn(-sc.omega, B.t[q], s);
+      }
+    if (sc.done) continue;
     auto val = [&](int64_t j, double *y) {
       for (int d = 0; d < MD; d++) {
         const int64_t q = S * j + d;
-        y[d] = B.r[q] + beta * po[q] + bo * vo[q];
+        const double r = __fma_rn(-sc.omega, B.t[q], B.s[q]);
+        y[d] = __fma_rn(bo, vo[q], __fma_rn(sc.beta, po[q], r));
       }
     };
     double acc[MD];
-    bi_row<MD>(B, i, g, val, acc);
-    if (g == 0 && it < B.n) {
+    row.times(B, g, val, acc);
+    if (own) {
       const uint8_t fl = B.flags[i];
       double y[MD];
       val(i, y);
@@ -418,88 +473,70 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k) {
         const double w = dof_fixed(fl, d, MD) ? y[d] : acc[d];
         pn[q] = y[d];
         vn[q] = w;
-        rv[0] += B.rhat[q] * w;
+        rv[0] = __fma_rn(B.rhat[q], w, rv[0]);
       }
     }
   }
-  bi_partials<1>(rv, B.part1);
+  if (!sc.done) bi_partials<1>(rv, B.part1);
 }
 
 template <int MD>
 __global__ void __launch_bounds__(kBiThreads) k_bi_shadow(const BiArgs B, int k) {
   constexpr int S = MD == 3 ? 4 : 2;
-  pdl_trigger_and_wait();
-  const BiScal in = B.sc[k & 1];
-  BiScal out = in;
-  double tot[1];
-  if (!in.done) {
-    bi_totals<1>(B.part1, B.np1, tot);
-    if (tot[0] == 0.)
-      out.done = 1;
-    else
-      out.alpha = in.rho / tot[0];
-  }
-  bi_store(B.sc + 2 + (k & 1), out);
-  if (out.done) return;
-  const double *v = B.v[k & 1];
+  __shared__ BiScal s_sc;
   const int g = threadIdx.x % kBiTeam;
-  double sums[3] = {};
-  constexpr int64_t R = kBiThreads / kBiTeam;
-  for (int64_t i0 = blockIdx.x * R; i0 < B.n; i0 += gridDim.x * R) {
-    const int64_t it = i0 + threadIdx.x / kBiTeam, i = it < B.n ? it : B.n - 1;
+  const int64_t first_row = blockIdx.x * kBiRows + threadIdx.x / kBiTeam;
+  BiRow<MD> row;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  row.fetch(B, min(first_row, B.n - 1), g);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (threadIdx.x < 32) {
+    BiScal sc = B.sc[k & 1];
+    double t[1];
+    bi_totals<1>(B.part1, t);
+    if (threadIdx.x == 0) {
+      if (!sc.done) {
+        if (t[0] == 0.)
+          sc.done = 1;  // breakdown: keep the iterate
+        else
+          sc.alpha = sc.rho / t[0];
+      }
+      s_sc = sc;
+      if (blockIdx.x == 0) B.sc[2 + (k & 1)] = sc;
+    }
+  }
+  __syncthreads();
+  const BiScal sc = s_sc;
+  if (sc.done) return;
+  const double *v = B.v[k & 1];
+  double sums[5] = {};
+  for (int64_t i0 = blockIdx.x * kBiRows; i0 < B.n; i0 += gridDim.x * kBiRows) {
+    const int64_t it = i0 + threadIdx.x / kBiTeam;
+    if (it != first_row) row.fetch(B, min(it, B.n - 1), g);
+    const int64_t i = row.i;
     auto val = [&](int64_t j, double *y) {
-      for (int d = 0; d < MD; d++) y[d] = B.r[S * j + d] + -out.alpha * v[S * j + d];
+      for (int d = 0; d < MD; d++) y[d] = __fma_rn(-sc.alpha, v[S * j + d], B.r[S * j + d]);
     };
     double acc[MD];
-    bi_row<MD>(B, i, g, val, acc);
+    row.times(B, g, val, acc);
     if (g == 0 && it < B.n) {
       const uint8_t fl = B.flags[i];
       double y[MD];
       val(i, y);
       for (int d = 0; d < MD; d++) {
         const int64_t q = S * i + d;
-        const double t = dof_fixed(fl, d, MD) ? y[d] : acc[d];
+        const double t = dof_fixed(fl, d, MD) ? y[d] : acc[d], h = B.rhat[q];
         B.s[q] = y[d];
         B.t[q] = t;
-        sums[0] += y[d] * y[d];
-        sums[1] += t * y[d];
-        sums[2] += t * t;
+        sums[0] = __fma_rn(y[d], y[d], sums[0]);
+        sums[1] = __fma_rn(t, y[d], sums[1]);
+        sums[2] = __fma_rn(t, t, sums[2]);
+        sums[3] = __fma_rn(h, y[d], sums[3]);
+        sums[4] = __fma_rn(h, t, sums[4]);
       }
     }
   }
-  bi_partials<3>(sums, B.part2);
-}
-
-__global__ void __launch_bounds__(kBiThreads) k_bi_update(const BiArgs B, int k) {
-  pdl_trigger_and_wait();
-  const BiScal in = B.sc[2 + (k & 1)];
-  BiScal out = in;
-  double tot[3];
-  bool half = false;
-  if (!in.done) {
-    bi_totals<3>(B.part2, B.np1, tot);
-    half = sqrt(tot[0]) <= in.stop || tot[2] == 0.;  // x += alpha p ends the solve
-    out.done = half;
-    out.omega = half ? 0. : tot[1] / tot[2];
-  }
-  bi_store(B.sc + 4 + (k & 1), out);
-  if (in.done) return;
-  const double *p = B.p[k & 1];
-  double sums[2] = {};
-  for (int64_t q = blockIdx.x * (int64_t)kBiThreads + threadIdx.x; q < B.m;
-       q += (int64_t)gridDim.x * kBiThreads) {
-    double x = B.x[q] + out.alpha * p[q];
-    if (!half) {
-      const double s = B.s[q];
-      x = x + out.omega * s;
-      const double r = s + -out.omega * B.t[q];
-      B.r[q] = r;
-      sums[0] += B.rhat[q] * r;
-      sums[1] += r * r;
-    }
-    B.x[q] = x;
-  }
-  bi_partials<2>(sums, B.part3);
+  bi_partials<5>(sums, B.part2);
 }
 
 // out = a x + b y + c z (any of y, z may be NULL).
@@ -588,11 +625,8 @@ cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim
   return cudaGetLastError();
 }
 
-void esqs_bicgstab_grid(int64_t n, int64_t m, BiArgs &B) {
-  B.np1 = (int)std::max<int64_t>(
-      1, std::min<int64_t>(kBiParts, (n * kBiTeam + kBiThreads - 1) / kBiThreads));
-  B.np3 = (int)std::max<int64_t>(1,
-                                 std::min<int64_t>(kBiParts, (m + kBiThreads - 1) / kBiThreads));
+int esqs_bicgstab_blocks(int64_t n) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kBiParts, (n + kBiRows - 1) / kBiRows));
 }
 
 // kBiGraph iterations as one CUDA graph (iteration parities 1, 0, 1, ...).
@@ -602,9 +636,8 @@ cudaError_t esqs_bicgstab_graph(const BiArgs &B, int mdim, cudaGraphExec_t *out,
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
   for (int k = 1; k <= kBiGraph && e == cudaSuccess; k++) {
-    e = launch_pdl(dir, B.np1, kBiThreads, 0, s, k > 1, B, k & 1);
-    if (e == cudaSuccess) e = launch_pdl(shadow, B.np1, kBiThreads, 0, s, true, B, k & 1);
-    if (e == cudaSuccess) e = launch_pdl(k_bi_update, B.np3, kBiThreads, 0, s, true, B, k & 1);
+    e = launch_pdl(dir, B.blocks, kBiThreads, 0, s, k > 1, B, k & 1);
+    if (e == cudaSuccess) e = launch_pdl(shadow, B.blocks, kBiThreads, 0, s, true, B, k & 1);
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(s, &g);
@@ -616,14 +649,13 @@ cudaError_t esqs_bicgstab_graph(const BiArgs &B, int mdim, cudaGraphExec_t *out,
 
 cudaError_t esqs_bicgstab(const BiArgs &B, cudaGraphExec_t graph, const double *rhs, int *iters,
                           cudaStream_t s) {
-  k_bi_init<<<B.np3, kBiThreads, 0, s>>>(B, rhs);
+  k_bi_init<<<B.blocks, kBiThreads, 0, s>>>(B, rhs);
   cudaError_t e = cudaGetLastError();
   BiScal st{};
-  // the state after each graph's last direction launch; max_iters ends the loop
-  while (e == cudaSuccess && !st.done && st.iters < B.max_iters) {
+  while (e == cudaSuccess && !st.done) {  // max_iters ends it on the device
     e = cudaGraphLaunch(graph, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&st, B.sc + 4, sizeof(st), cudaMemcpyDeviceToHost, s);
+      e = cudaMemcpyAsync(&st, B.sc + 2, sizeof(st), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
   *iters = st.iters;

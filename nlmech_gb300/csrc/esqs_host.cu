@@ -113,9 +113,8 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
                        &bi.p[1], &bi.v[0], &bi.v[1], &bi.s, &bi.t})
     if (e == cudaSuccess) e = q->alloc(ptr, q->m);
   if (e == cudaSuccess) e = q->alloc(&bi.part1, kBiParts);
-  if (e == cudaSuccess) e = q->alloc(&bi.part2, 3 * kBiParts);
-  if (e == cudaSuccess) e = q->alloc(&bi.part3, 2 * kBiParts);
-  if (e == cudaSuccess) e = q->alloc(&bi.sc, 6);
+  if (e == cudaSuccess) e = q->alloc(&bi.part2, 5 * kBiParts);
+  if (e == cudaSuccess) e = q->alloc(&bi.sc, 4);
   const size_t md = (size_t)q->mdim;
   if (e == cudaSuccess) e = q->alloc(&q->J, md * md * q->nblocks);
   if (e == cudaSuccess) e = q->alloc(&q->bond, (3 * md + md * md) * (size_t)h->nnz);
@@ -133,7 +132,7 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   bi.x = q->dx;
   bi.tol = prm->lin_tol;
   bi.max_iters = prm->lin_max_iters;
-  esqs_bicgstab_grid(h->n, q->m, bi);
+  bi.blocks = esqs_bicgstab_blocks(h->n);
   if (e == cudaSuccess) e = cudaMemsetAsync(q->body, 0, sizeof(double) * q->m, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {

@@ -25,13 +25,13 @@ cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim
                           const double *u, const double *theta, double eps, int64_t nnz,
                           const int *rows, const int *ocols, double *bond, double *J,
                           cudaStream_t s);
-// BiCGSTAB state on the device (sc: two slots, by iteration parity, for each of
-// the three launches of an iteration).
+// BiCGSTAB state on the device (sc: slots 0-1 written by the direction launch,
+// 2-3 by the shadow launch, by iteration parity).
 struct BiScal {
-  double rho, alpha, omega, stop;
+  double rho, alpha, omega, beta, stop2;
   int done, iters;
 };
-constexpr int kBiParts = 512;  // most blocks of a launch
+constexpr int kBiParts = 1216;  // most blocks of a launch (8 per SM)
 struct BiArgs {
   int64_t n, m;             // nodes, entries of a vector (S per node)
   const uint8_t *flags;
@@ -39,14 +39,14 @@ struct BiArgs {
   const int *cols;
   const double *J;
   double *r, *rhat, *p[2], *v[2], *s, *t, *x;
-  double *part1, *part2, *part3;  // kBiParts, 3 and 2 times kBiParts doubles
-  int np1, np3;                   // blocks of the product and update launches
-  BiScal *sc;                     // 6
-  double tol;                     // ||r|| <= tol ||rhs||
+  double *part1, *part2;    // kBiParts and 5 kBiParts doubles
+  int blocks;
+  BiScal *sc;               // 4
+  double tol;               // ||r|| <= tol ||rhs||
   int max_iters;
 };
 constexpr int kBiGraph = 32;  // iterations per graph launch (even)
-void esqs_bicgstab_grid(int64_t n, int64_t m, BiArgs &B);
+int esqs_bicgstab_blocks(int64_t n);
 cudaError_t esqs_bicgstab_graph(const BiArgs &B, int mdim, cudaGraphExec_t *out, cudaStream_t s);
 // J x = rhs; synchronises.
 cudaError_t esqs_bicgstab(const BiArgs &B, cudaGraphExec_t graph, const double *rhs, int *iters,

@@ -41,51 +41,60 @@ __device__ __forceinline__ double esqs_t(const StepParams &P, int mdim, double m
   return mdim == 2 ? es_t64<2>(P, mi, th, e, Xl) : es_t64<3>(P, mi, th, e, Xl);
 }
 
-// Dilatation theta_i (stateBasedHelperFunctions.cpp:26-83, every bond):
-// theta_i = sum_j (c / m_i) f2 |X| e omega V_j, c = mdim, f2 = factor2D in 2-D.
-template <int SD>
-__device__ double theta_node(const StepParams &P, const DevPtrs &D, int mdim, const double *u,
-                             int64_t i) {
+// Dilatations and forces: G lanes per node (1 or 8) evaluate the bonds of a
+// group of G side by side, and their terms are added in row order.  With one
+// thread per node a 1,440-node plate keeps one warp in flight on 45 SMs:
+// 60 + 162 us for the two kernels, 14 + 39 us with 8 lanes.
+
+// theta_i = sum_j (c / m_i) f2 |X| e omega V_j over every bond, c = mdim, f2 =
+// factor2D in 2-D (stateBasedHelperFunctions.cpp:26-83).
+template <int SD, int G>
+__global__ void __launch_bounds__(128)
+    k_esqs_theta(const StepParams P, const DevPtrs D, int mdim, const double *u, double *theta) {
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  if (i >= P.n) return;
+  const int c = threadIdx.x % G;
+  const unsigned team = G == 1 ? 0u : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G);
   double xi[3], ui[3];
   ld_node<SD>(D.pos64, i, xi);
   ld_node_rw<SD>(u, i, ui);
-  const double mi = D.mw64[i];
-  const double c = (double)mdim;
+  const double cm = (double)mdim / D.mw64[i] * (mdim == 2 ? P.es_factor2D : 1.) * 1.;
+  const int64_t r0 = D.rowptr[i];
+  const int len = (int)(D.rowptr[i + 1] - r0);
   double th = 0.;
-  for (int64_t k = D.rowptr[i]; k < D.rowptr[i + 1]; k++) {
-    const int j = D.cols[k];
+  for (int kb = 0; kb < len; kb += G) {
+    const int j = D.cols[r0 + min(kb + c, len - 1)];
     double xj[3], uj[3], Y[3], Xl, e;
     ld_node<SD>(D.pos64, j, xj);
     ld_node_rw<SD>(u, j, uj);
     es_geom64<SD>(xi, ui, xj, uj, Y, Xl, e);
-    if (mdim == 2)
-      th += (c / mi) * P.es_factor2D * 1. * Xl * e * es_omega(P, Xl) * D.vol64[j];
-    else
-      th += (c / mi) * 1. * Xl * e * es_omega(P, Xl) * D.vol64[j];
+    const double t = cm * Xl * e * es_omega(P, Xl) * D.vol64[j];
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      const double q = G == 1 ? t : __shfl_sync(team, t, g, G);
+      if (kb + g < len) th += q;
+    }
   }
-  return th;
+  if (c == 0) theta[i] = th;
 }
 
-template <int SD>
-__global__ void k_esqs_theta(const StepParams P, const DevPtrs D, int mdim, const double *u,
-                             double *theta) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+template <int SD, int G>
+__global__ void __launch_bounds__(128)
+    k_esqs_force(const StepParams P, const DevPtrs D, int mdim, const double *u,
+                 const double *theta, double *f) {
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   if (i >= P.n) return;
-  theta[i] = theta_node<SD>(P, D, mdim, u, i);
-}
-
-template <int SD>
-__global__ void k_esqs_force(const StepParams P, const DevPtrs D, int mdim, const double *u,
-                             const double *theta, double *f) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
+  const int c = threadIdx.x % G;
+  const unsigned team = G == 1 ? 0u : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G);
   double xi[3], ui[3];
   ld_node<SD>(D.pos64, i, xi);
   ld_node_rw<SD>(u, i, ui);
   const double mi = D.mw64[i], thi = theta[i];
+  const int64_t r0 = D.rowptr[i];
+  const int len = (int)(D.rowptr[i + 1] - r0);
   double fi[3] = {0., 0., 0.};
-  for (int64_t k = D.rowptr[i]; k < D.rowptr[i + 1]; k++) {
-    const int j = D.cols[k];
+  for (int kb = 0; kb < len; kb += G) {
+    const int j = D.cols[r0 + min(kb + c, len - 1)];
     double xj[3], uj[3], Y[3], Xl, e;
     ld_node<SD>(D.pos64, j, xj);
     ld_node_rw<SD>(u, j, uj);
@@ -93,9 +102,16 @@ __global__ void k_esqs_force(const StepParams P, const DevPtrs D, int mdim, cons
     const double Yl = sqrt(Y[0] * Y[0] + Y[1] * Y[1] + Y[2] * Y[2]);
     const double tsum = esqs_t(P, mdim, mi, thi, e, Xl) + esqs_t(P, mdim, D.mw64[j], theta[j], e, Xl);
     const double s = tsum * es_omega(P, Xl) * D.vol64[j];
-    for (int d = 0; d < 3; d++) fi[d] = fi[d] + (Y[d] / Yl) * s;
+    for (int d = 0; d < SD; d++) {
+      const double t = (Y[d] / Yl) * s;
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const double q = G == 1 ? t : __shfl_sync(team, t, g, G);
+        if (kb + g < len) fi[d] = fi[d] + q;
+      }
+    }
   }
-  st_node<SD>(f, i, fi);
+  if (c == 0) st_node<SD>(f, i, fi);
 }
 
 // r = f + b on free dofs, 0 on fixed ones (QuasiStaticModel::computeResidual,
@@ -197,56 +213,57 @@ __device__ __forceinline__ int row_find(const int64_t *rowptr, const int *ocols,
   return lo < end && ocols[lo] == key ? (int)(lo - r0) : -1;
 }
 
-// A warp per row node i, its lanes over the blocks b (b = 0: i itself, b = 1 +
-// k: the k-th neighbour).  full = 0 keeps the (i, rr; j, rr) entries only, as
-// the reference does; full = 1 whole blocks.  Block b of row i is row-major at
-// J[mdim^2 (rowptr[i] + i + b)]; rows and columns of fixed dofs are zero.
+// Sums over a row's bonds, in one fixed order: sum B, sum dF/dtheta_i, sum A.
+// A warp per row.
 template <int MD>
 __global__ void __launch_bounds__(128)
-    k_esqs_rows(int64_t n, const DevPtrs D, int full, const int *ocols, const double *bond,
-                double *J) {
-  constexpr int R = 3 * MD + MD * MD;
+    k_esqs_sums(int64_t n, const int64_t *rowptr, const double *bond, double *sums) {
+  constexpr int R = 3 * MD + MD * MD, Q = 2 * MD + MD * MD;
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;
   const int lane = threadIdx.x & 31;
+  double v[Q] = {};
+  for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += 32) {
+    const double *o = bond + R * q;
+    for (int d = 0; d < MD; d++) v[d] += o[d];
+    for (int d = 0; d < MD + MD * MD; d++) v[MD + d] += o[2 * MD + d];
+  }
+  for (int s = 16; s > 0; s >>= 1)
+    for (int d = 0; d < Q; d++) v[d] += __shfl_xor_sync(0xffffffffu, v[d], s);
+  if (lane == 0)
+    for (int d = 0; d < Q; d++) sums[Q * i + d] = v[d];
+}
+
+// A block of four warps per row node i: lanes over the blocks b (b = 0: i
+// itself, b = 1 + k: the k-th neighbour), warps over the neighbours k whose
+// dilatation u_j moves (the search of j in row k is a chain of loads: one warp
+// per row took 196 us for 1,440 rows, 35 us with four).  full = 0 keeps
+// the (i, rr; j, rr) entries only, as the reference does; full = 1 whole
+// blocks.  Block b of row i is row-major at J[mdim^2 (rowptr[i] + i + b)]; rows
+// and columns of fixed dofs are zero.
+template <int MD>
+__global__ void __launch_bounds__(128)
+    k_esqs_rows(const DevPtrs D, int full, const int *ocols, const double *bond,
+                const double *sums, double *J) {
+  constexpr int R = 3 * MD + MD * MD, Q = 2 * MD + MD * MD, M2 = MD * MD;
+  __shared__ double part[3][M2][32];
+  const int64_t i = blockIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t r0 = D.rowptr[i];
   const int len = (int)(D.rowptr[i + 1] - r0);
-  // sums over the row, in one fixed order
-  double G[MD] = {}, C[MD] = {}, A[MD * MD] = {};
-  for (int k = lane; k < len; k += 32) {
-    const double *o = bond + R * (r0 + k);
-    for (int d = 0; d < MD; d++) {
-      C[d] += o[d];
-      G[d] += o[2 * MD + d];
-    }
-    for (int d = 0; d < MD * MD; d++) A[d] += o[3 * MD + d];
-  }
-  for (int s = 16; s > 0; s >>= 1) {
-    for (int d = 0; d < MD; d++) {
-      C[d] += __shfl_xor_sync(0xffffffffu, C[d], s);
-      G[d] += __shfl_xor_sync(0xffffffffu, G[d], s);
-    }
-    for (int d = 0; d < MD * MD; d++) A[d] += __shfl_xor_sync(0xffffffffu, A[d], s);
-  }
+  const double *C = sums + Q * i, *G = C + MD, *A = C + 2 * MD;
   const uint8_t fli = D.flags[i];
-  for (int b = lane; b <= len; b += 32) {
-    const int64_t j = b == 0 ? i : (int64_t)D.cols[r0 + b - 1];
+  for (int b0 = 0; b0 <= len; b0 += 32) {
+    const int b = b0 + lane;
+    const bool in = b <= len;
+    const int64_t j = in && b > 0 ? (int64_t)D.cols[r0 + b - 1] : i;
     const int key = D.perm_dev[j];
-    double acc[MD * MD];
-    {
-      const double *o = bond + R * (r0 + b - 1);
-      for (int ss = 0; ss < MD; ss++)
-        for (int rr = 0; rr < MD; rr++)
-          acc[ss * MD + rr] = b == 0 ? -A[ss * MD + rr] - G[ss] * C[rr]
-                                     : o[3 * MD + ss * MD + rr] + G[ss] * o[rr];
-    }
-    for (int k = 0; k < len; k++) {
+    double acc[M2] = {};
+    for (int k = w; in && k < len; k += 4) {
       const int64_t kn = D.cols[r0 + k];
       double dth[MD];
       if (kn == j) {
-        for (int d = 0; d < MD; d++) dth[d] = 0.;
-        for (int64_t q = D.rowptr[kn]; q < D.rowptr[kn + 1]; q++)
-          for (int d = 0; d < MD; d++) dth[d] -= bond[R * q + d];
+        for (int d = 0; d < MD; d++) dth[d] = -sums[Q * kn + d];
       } else {
         const int p = row_find(D.rowptr, ocols, kn, key);
         if (p < 0) continue;
@@ -256,13 +273,23 @@ __global__ void __launch_bounds__(128)
       for (int ss = 0; ss < MD; ss++)
         for (int rr = 0; rr < MD; rr++) acc[ss * MD + rr] += h[ss] * dth[rr];
     }
-    const uint8_t flj = D.flags[j];
-    double *blk = J + MD * MD * (r0 + i + b);
-    for (int ss = 0; ss < MD; ss++)
-      for (int rr = 0; rr < MD; rr++) {
-        const bool on = (full || ss == rr) && !dof_fixed(fli, ss, MD) && !dof_fixed(flj, rr, MD);
-        blk[ss * MD + rr] = on ? acc[ss * MD + rr] : 0.;
-      }
+    if (w > 0)
+      for (int d = 0; d < M2; d++) part[w - 1][d][lane] = acc[d];
+    __syncthreads();
+    if (w == 0 && in) {
+      const uint8_t flj = D.flags[j];
+      double *blk = J + M2 * (r0 + i + b);
+      const double *o = bond + R * (r0 + (b > 0 ? b - 1 : 0));
+      for (int ss = 0; ss < MD; ss++)
+        for (int rr = 0; rr < MD; rr++) {
+          const int d = ss * MD + rr;
+          const double own = b == 0 ? -A[d] - G[ss] * C[rr] : o[3 * MD + d] + G[ss] * o[rr];
+          const double v = own + acc[d] + part[0][d][lane] + part[1][d][lane] + part[2][d][lane];
+          const bool on = (full || ss == rr) && !dof_fixed(fli, ss, MD) && !dof_fixed(flj, rr, MD);
+          blk[d] = on ? v : 0.;
+        }
+    }
+    __syncthreads();
   }
 }
 
@@ -579,14 +606,15 @@ unsigned blocks_of(int64_t m, int bs) { return (unsigned)((m + bs - 1) / bs); }
 cudaError_t esqs_force(const StepParams &P, const DevPtrs &D, int S, int mdim, const double *u,
                        double *theta, double *f, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  const unsigned g = blocks_of(P.n, 128);
-  if (S == 2) {
-    k_esqs_theta<2><<<g, 128, 0, s>>>(P, D, mdim, u, theta);
-    k_esqs_force<2><<<g, 128, 0, s>>>(P, D, mdim, u, theta, f);
-  } else {
-    k_esqs_theta<3><<<g, 128, 0, s>>>(P, D, mdim, u, theta);
-    k_esqs_force<3><<<g, 128, 0, s>>>(P, D, mdim, u, theta, f);
-  }
+  // teams below 16384 nodes, where one thread per node leaves SMs idle
+  const int G = P.n < 16384 ? 8 : 1;
+  const unsigned g = blocks_of(P.n * G, 128);
+  (S == 2 ? (G == 1 ? k_esqs_theta<2, 1> : k_esqs_theta<2, 8>)
+          : (G == 1 ? k_esqs_theta<3, 1> : k_esqs_theta<3, 8>))<<<g, 128, 0, s>>>(P, D, mdim, u,
+                                                                                 theta);
+  (S == 2 ? (G == 1 ? k_esqs_force<2, 1> : k_esqs_force<2, 8>)
+          : (G == 1 ? k_esqs_force<3, 1> : k_esqs_force<3, 8>))<<<g, 128, 0, s>>>(P, D, mdim, u,
+                                                                                 theta, f);
   return cudaGetLastError();
 }
 
@@ -610,18 +638,21 @@ cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *rows, int 
 
 cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim, int full,
                           const double *u, const double *theta, double eps, int64_t nnz,
-                          const int *rows, const int *ocols, double *bond, double *J,
-                          cudaStream_t s) {
+                          const int *rows, const int *ocols, double *bond, double *sums,
+                          double *J, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
   if (nnz > 0) {
     const unsigned g = blocks_of(nnz, 128);
     (S == 2 ? k_esqs_bonds<2> : k_esqs_bonds<3>)<<<g, 128, 0, s>>>(P, D, mdim, rows, nnz, u, theta,
                                                                    eps, bond);
   }
+  (mdim == 1   ? k_esqs_sums<1>
+   : mdim == 2 ? k_esqs_sums<2>
+               : k_esqs_sums<3>)<<<blocks_of(32 * P.n, 128), 128, 0, s>>>(P.n, D.rowptr, bond,
+                                                                          sums);
   (mdim == 1   ? k_esqs_rows<1>
    : mdim == 2 ? k_esqs_rows<2>
-               : k_esqs_rows<3>)<<<blocks_of(32 * P.n, 128), 128, 0, s>>>(P.n, D, full, ocols,
-                                                                          bond, J);
+               : k_esqs_rows<3>)<<<(unsigned)P.n, 128, 0, s>>>(D, full, ocols, bond, sums, J);
   return cudaGetLastError();
 }
 

@@ -427,17 +427,19 @@ typedef struct nlm_qs_params {
   double guess_accept; /* a guess is used only if its linearised residual is
                           at most guess_accept times that of the plain
                           start (<= 0: 0.1)                                  */
-  int krylov_launch;   /* 0: the FP32 Krylov solve runs two launches per
-                          iteration (default; 46.6 us per iteration with the
-                          Newton work around it on the 200 x 200 plate);
-                          1: one cooperative launch per solve with grid
-                          barriers between its phases where the device
-                          allows it (50.2 us per iteration there)          */
-  double wait_limit_s; /* bound of each grid-barrier wait of that launch
-                          (<= 0: 1 s); a wait that runs out ends the solve
-                          with NLM_ERR_TIMEOUT and the handle stays usable   */
-  int barrier_extra;   /* testing the bound only: arrivals each barrier waits
-                          for beyond the launched blocks (0 in use; > 0 makes
+  int krylov_launch;   /* 0: the FP32 Krylov solve runs in one cooperative
+                          launch where the device allows it and the tangent
+                          fits the SMs' shared memory (up to about 1.8 million
+                          2-D bonds), else in two launches per iteration;
+                          200 x 200 plate: 7 us per iteration against 27
+                          1: the same, but a wait of that launch that runs out
+                          is an error instead of a change to two launches   */
+  double wait_limit_s; /* bound of each grid-wide wait of that launch
+                          (<= 0: 1 s); a wait that runs out ends the launch;
+                          with krylov_launch = 1 the load step then fails with
+                          NLM_ERR_TIMEOUT and the handle stays usable        */
+  int barrier_extra;   /* testing the bound only: arrivals each wait counts
+                          beyond the launched blocks (0 in use; > 0 makes
                           every wait run out)                                */
   double lin_tol_gamma; /* > 0: a Newton iteration whose residual is already
                           near the target solves to the looser relative

@@ -30,9 +30,11 @@
 // are left out of the tangent so the preconditioned CG matrix stays SPD.
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "fd_internal.h"
+#include "fp32_common.cuh"
 #include "qs_internal.h"
 #include "state_io.cuh"
 
@@ -202,6 +204,22 @@ __device__ __forceinline__ void block_jacobi(const T *b, uint8_t fl, const T rv[
         zv[c] = (inv[3 * c] * rv[0] + inv[3 * c + 1] * rv[1] + inv[3 * c + 2] * rv[2]) / det;
     }
   }
+}
+
+// Packed inverse of a node's diagonal block for the FP32 solves, formed in FP64
+// (the determinant of a 3-D block, about 1e54 at h = 5e-4 m, is past FP32's
+// range); zero rows and columns for fixed dofs.
+template <int DIM>
+__device__ __forceinline__ void inv_diag32(const double *b, uint8_t fl, float *mi) {
+  double inv[3][3];
+  for (int c = 0; c < DIM; c++) {
+    const double e[3] = {c == 0 ? 1. : 0., c == 1 ? 1. : 0., c == 2 ? 1. : 0.};
+    block_jacobi<DIM, double>(b, fl, e, inv[c]);
+  }
+  int q = 0;
+  for (int c = 0; c < DIM; c++)
+    for (int d = 0; d <= c; d++, q++)
+      mi[q] = (fl >> c & 1) || (fl >> d & 1) ? 0.f : (float)inv[c][d];
 }
 
 // Block-Jacobi preconditioner: z_i = (D_i)^-1 r_i on the free dofs of node i
@@ -490,19 +508,24 @@ __device__ __forceinline__ void block_sum2_f(float va, float vb, double *pa, dou
 }
 
 template <int DIM>
-__global__ void k_qs_precond32(int64_t n, const uint8_t *flags, const float *dblk,
-                               const float *r, float *z, double *part) {
+__global__ void k_inv_diag32(int64_t n, const uint8_t *flags, const double *dblk, float *minv) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  constexpr int NB = DIM == 2 ? 3 : 6;
+  if (i < n) inv_diag32<DIM>(dblk + NB * i, flags[i], minv + NB * i);
+}
+
+template <int DIM>
+__global__ void k_qs_precond32(int64_t n, const float *minv, const float *r, float *z,
+                               double *part) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   constexpr int NB = DIM == 2 ? 3 : 6;
   float dot = 0.f;
   if (i < n) {
-    const uint8_t fl = flags[i];
-    float rv[3] = {0.f, 0.f, 0.f}, zv[3];
-    for (int c = 0; c < DIM; c++) rv[c] = (fl >> c & 1) ? 0.f : r[DIM * i + c];
-    block_jacobi<DIM, float>(dblk + NB * i, fl, rv, zv);
+    float zv[3];
+    sym_mul<float>(DIM, minv + NB * i, r + DIM * i, zv);
     for (int c = 0; c < DIM; c++) {
       z[DIM * i + c] = zv[c];
-      dot = fmaf(rv[c], zv[c], dot);
+      dot = fmaf(r[DIM * i + c], zv[c], dot);
     }
   }
   block_sum_f(dot, part);
@@ -586,7 +609,7 @@ __global__ void __launch_bounds__(256) k_cg32_dir_spmv(
 // FP32 form of the second CG launch (see k_cg_update).  Its last block forms
 // beta_k = rz_{k+1} / rz_k for the next first launch.
 template <int DIM>
-__global__ void k_cg32_update(int64_t n, const uint8_t *flags, const float *dblk, const float *p,
+__global__ void k_cg32_update(int64_t n, const float *minv, const float *p,
                               const float *ap, float *x, float *r, float *z,
                               const double *rz_cur, double *rz_part, double *rr_part,
                               unsigned *ticket, double *rz_next, double *rr_total, float *fs) {
@@ -595,17 +618,15 @@ __global__ void k_cg32_update(int64_t n, const uint8_t *flags, const float *dblk
   constexpr int NB = DIM == 2 ? 3 : 6;
   float drz = 0.f, drr = 0.f;
   if (i < n) {
-    const uint8_t fl = flags[i];
     float rv[3] = {0.f, 0.f, 0.f}, zv[3] = {0.f, 0.f, 0.f};
     for (int c = 0; c < DIM; c++) {
       const int64_t k = DIM * i + c;
       x[k] = fmaf(alpha, p[k], x[k]);
-      const float rk = fmaf(-alpha, ap[k], r[k]);
-      r[k] = rk;
-      drr = fmaf(rk, rk, drr);
-      rv[c] = (fl >> c & 1) ? 0.f : rk;
+      rv[c] = fmaf(-alpha, ap[k], r[k]);
+      r[k] = rv[c];
+      drr = fmaf(rv[c], rv[c], drr);
     }
-    block_jacobi<DIM, float>(dblk + NB * i, fl, rv, zv);
+    sym_mul<float>(DIM, minv + NB * i, rv, zv);
     for (int c = 0; c < DIM; c++) {
       z[DIM * i + c] = zv[c];
       drz = fmaf(rv[c], zv[c], drz);
@@ -622,195 +643,340 @@ __global__ void k_cg32_update(int64_t n, const uint8_t *flags, const float *dblk
 }
 
 // ---- the FP32 PCG in one cooperative launch -------------------------------
-// The two-launch iteration above costs two kernel launches per iteration and
-// a host round trip every few iterations; at 40,000 nodes that, not the
-// work, sets the iteration time.  k_cg32_coop runs the whole solve in one
-// launch whose blocks are all resident (cudaLaunchCooperativeKernel): each
-// iteration is the same two phases separated by a grid barrier, and every
-// block forms alpha, beta and the convergence test itself from the block
-// partials, summed in one fixed order (so every block takes the same
-// decision and the result does not depend on timing).
-//
-// Grid barrier: an arrival counter and a generation word.  A waiting block
-// polls the generation with a bounded wait (wait_ns of globaltimer); a wait
-// that runs out sets status = NLM_ERR_TIMEOUT, and every block leaves at its
-// next barrier once status is set, so the launch always ends.  expect is the
-// number of arrivals a barrier completes on: gridDim.x in use (more only to
-// test the bound).
+// At 40,000 nodes the two-launch iteration (27 us: 16.4 + 9.7) is bound by the
+// launches, the last-block sums and re-reading the tangent from L2, not by the
+// 21 MB it moves.  k_cg32_res runs the whole solve in one launch of one block
+// per SM, all resident (cudaLaunchCooperativeKernel), and keeps what a block
+// needs on its SM: each block owns a range of consecutive nodes; their tangent
+// blocks sit in shared memory with the neighbour's local id (16 bytes per 2-D
+// bond, read once per solve), x, r, z and the inverse diagonal block of a node
+// in the registers of one thread, and the search direction of the block's
+// nodes and of their halo in shared memory, so that an iteration reads nothing
+// but the halo's new z.  Halo lists and local ids are laid out once, at
+// creation (k_cg_res_setup).
+// The two sums of an iteration: a block stores its partial (FP32, as in the
+// two-launch form) with the iteration number in one 8-byte word, counts itself
+// in, waits for the count and adds all blocks' words in one fixed order, so
+// every block forms the same alpha, beta and convergence decision.  A word whose
+// number is not yet this iteration's is read again, so only z, which the other
+// blocks read after the second sum, needs a fence before the count.  The words
+// are added and the step lengths divided in double-float (two-sum) arithmetic:
+// an FP64 add takes 67 cycles here, a division 566, and they sit on the one
+// chain everything waits for.  (152 SMs polling each other's words instead of
+// one counter took 7,500 cycles per sum, with one array or with a private
+// mailbox per block alike; the counter and the read 3,400.)
+// A poll is bounded (wait_ns of globaltimer); one that runs out sets status =
+// NLM_ERR_TIMEOUT and every block leaves at its next poll, so the launch
+// always ends.  200 x 200 plate, horizon 3h: 7 us per iteration, of which the
+// two sums take 4 (counting in, the skew of the blocks, reading the words), the
+// product 1.4 and the halo 0.8; a load step 38.0 -> 13.7 ms.
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
 
-// coop[0] arrivals, coop[1] generation, coop[2] status
-__device__ bool coop_barrier(unsigned *coop, unsigned expect, uint64_t wait_ns) {
-  __shared__ int s_ok;
+constexpr int kResThreads = 1024;
+constexpr int kResHash = 2 * kResHalo;
+
+// Halo list (ids of the nodes outside the block's range that its rows meet)
+// and, per bond, the local id of its neighbour: own nodes first, then the
+// halo.  nh < 0: more than kResHalo of them.
+__global__ void __launch_bounds__(kResThreads)
+    k_cg_res_setup(int64_t n, int nb, const int64_t *rowptr, const int *cols, int *halo, int *nh,
+                   uint16_t *lid) {
+  __shared__ int keys[kResHash], vals[kResHash], count;
+  const int64_t n0 = (int64_t)blockIdx.x * nb, n1 = min(n0 + nb, n);
+  for (int k = threadIdx.x; k < kResHash; k += kResThreads) keys[k] = -1;
+  if (threadIdx.x == 0) count = 0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned *gen = coop + 1;
-    volatile int *status = reinterpret_cast<volatile int *>(coop + 2);
-    const unsigned g = *gen;
-    __threadfence();
-    int ok = 1;
-    if (atomicAdd(coop, 1u) == expect - 1) {
-      atomicExch(coop, 0u);
-      __threadfence();
-      atomicAdd(coop + 1, 1u);
-    } else {
-      const uint64_t t0 = globaltimer_ns();
-      while (*gen == g) {
-        if (*status != 0) {
-          ok = 0;
-          break;
-        }
-        if (globaltimer_ns() - t0 > wait_ns) {
-          atomicExch(reinterpret_cast<int *>(coop + 2), NLM_ERR_TIMEOUT);
-          ok = 0;
-          break;
-        }
-        __nanosleep(100);
+  auto slot_of = [&](int j) { return (int)(((unsigned)j * 2654435761u) >> 16) % kResHash; };
+  const int64_t q0 = rowptr[n0], q1 = rowptr[n1];
+  for (int64_t q = q0 + threadIdx.x; q < q1; q += kResThreads) {
+    const int j = cols[q];
+    if (j >= n0 && j < n1) continue;
+    int s = slot_of(j);
+    for (int t = 0; t < kResHash; t++, s = (s + 1) % kResHash) {
+      const int old = atomicCAS(keys + s, -1, j);
+      if (old == j) break;
+      if (old == -1) {
+        const int k = atomicAdd(&count, 1);
+        vals[s] = k;
+        if (k < kResHalo) halo[blockIdx.x * kResHalo + k] = j;
+        break;
       }
     }
-    __threadfence();
-    if (*status != 0) ok = 0;
-    s_ok = ok;
   }
   __syncthreads();
-  return s_ok != 0;
+  if (threadIdx.x == 0) nh[blockIdx.x] = count <= kResHalo ? count : -1;
+  if (count > kResHalo) return;
+  for (int64_t q = q0 + threadIdx.x; q < q1; q += kResThreads) {
+    const int j = cols[q];
+    int id = (int)(j - n0);
+    if (j < n0 || j >= n1) {
+      int s = slot_of(j);
+      while (keys[s] != j) s = (s + 1) % kResHash;  // present
+      id = nb + vals[s];
+    }
+    lid[q] = (uint16_t)id;
+  }
 }
 
-// Sum of part[0 .. nb) in a fixed order, the same in every block.
-__device__ double coop_sum(const double *part, int nb) {
-  __shared__ double sh[32];
-  double v = 0.;
-  for (int k = threadIdx.x; k < nb; k += blockDim.x) v += __ldcg(part + k);
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// Warp 0: publish N partials, wait for all blocks, sum their words in one fixed
+// order; false when a wait ran out or another block gave up.  fence: what the
+// block wrote before is visible to a block that has returned.
+template <int N, bool FENCE>
+__device__ __forceinline__ bool res_sum(const CgRes &A, int slot, uint32_t epoch, uint32_t arrivals,
+                                        const float v[N], df sum[N]) {
+  const int lane = threadIdx.x;
+  bool ok = true;
+  if (lane == 0) {
+    if (FENCE) __threadfence();
+    for (int a = 0; a < N; a++)
+      *(volatile unsigned long long *)(A.words + (slot + a) * A.stride + blockIdx.x) =
+          ((unsigned long long)epoch << 32) | __float_as_uint(v[a]);
+    atomicAdd(A.count, 1u);
+  }
+  uint64_t t0 = 0;
+  int polls = 0;
+  // the time and the other blocks' status every 64 polls
+  auto give_up = [&]() {
+    if ((++polls & 63) == 0) {
+      if (*(volatile const int *)A.status != 0) return true;
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > A.wait_ns) {
+        atomicExch(A.status, NLM_ERR_TIMEOUT);
+        return true;
+      }
+    }
+    return false;
+  };
+  if (lane == 0)
+    while (ok && *(volatile const unsigned *)A.count < arrivals) ok = !give_up();
+  ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+  if (FENCE) __threadfence();
+  for (int a = 0; a < N; a++) sum[a] = df{0.f, 0.f};
+  for (int b0 = lane; b0 < A.blocks; b0 += 160) {
+    unsigned long long w[5][N];
+    bool all = true;
+    do {
+      all = true;
+#pragma unroll
+      for (int u = 0; u < 5; u++)
+#pragma unroll
+        for (int a = 0; a < N; a++) {
+          const int b = min(b0 + 32 * u, A.blocks - 1);
+          w[u][a] = *(volatile const unsigned long long *)(A.words + (slot + a) * A.stride + b);
+          all = all && (uint32_t)(w[u][a] >> 32) == epoch;
+        }
+      if (!all && ok) ok = !give_up();
+    } while (!all && ok);
+#pragma unroll
+    for (int u = 0; u < 5; u++)
+#pragma unroll
+      for (int a = 0; a < N; a++)
+        if (b0 + 32 * u < A.blocks)
+          sum[a] = df_add(sum[a], df{__uint_as_float((uint32_t)w[u][a]), 0.f});
+  }
+  ok = __all_sync(0xffffffffu, ok);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      const df q{__shfl_xor_sync(0xffffffffu, sum[a].hi, o),
+                 __shfl_xor_sync(0xffffffffu, sum[a].lo, o)};
+      sum[a] = df_add(sum[a], q);
+    }
+  return ok;
+}
+
+// a / b rounded to FP32 (a quotient of the leading parts and its correction).
+__device__ __forceinline__ float df_div(df a, df b) {
+  const float q = __fdiv_rn(a.hi, b.hi);
+  const float r = fmaf(-q, b.hi, a.hi) + fmaf(-q, b.lo, a.lo);
+  const float c = __fdiv_rn(r, b.hi);
+  return isfinite(c) ? q + c : q;
+}
+
+// Block sums of N floats; warp 0's lanes end with them.  Ends with warp 0
+// alone past a block barrier.
+template <int N>
+__device__ __forceinline__ void res_block_sum(float v[N], float (*sh)[32]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int a = 0; a < N; a++) v[a] += __shfl_xor_sync(0xffffffffu, v[a], o);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0)
+    for (int a = 0; a < N; a++) sh[a][w] = v[a];
   __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0.;
-  for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += sh[k];
-  return t;
+  if (w == 0) {
+    for (int a = 0; a < N; a++) v[a] = sh[a][l];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int a = 0; a < N; a++) v[a] += __shfl_xor_sync(0xffffffffu, v[a], o);
+  }
 }
 
-constexpr int kCoopThreads = 256;
-
-// res[0] = iterations done, res[1] = r.r at the end
+// res[0] = iterations done, res[1] = r.r at the end, res[2] = its target
 template <int DIM>
-__global__ void __launch_bounds__(256) k_cg32_coop(
-    int64_t n, const uint8_t *flags, const int64_t *rowptr, const int *cols, const float *blk,
-    const float *dblk, float *p0, float *p1, float *ap, float *x, float *r, float *z,
-    double *part, const double *rz0, double target, int max_iters, unsigned *coop,
-    unsigned expect, uint64_t wait_ns, double *res) {
+__global__ void __launch_bounds__(kResThreads, 1) k_cg32_res(const CgRes A) {
   constexpr int NB = DIM == 2 ? 3 : 6;
-  constexpr int NP = DIM == 2 ? 4 : 8;
-  const int G = (int)gridDim.x;
-  double *pap_p = part, *rz_p = part + G, *rr_p = part + 2 * G;
-  double rz = *rz0, rr = 0.;
+  constexpr int NW = DIM == 2 ? 1 : 2;  // float4 words per bond
+  extern __shared__ float4 s_bond[];
+  __shared__ float s_red[2][32];
+  __shared__ float s_scal;
+  __shared__ int s_stop;
+  const int64_t n0 = (int64_t)blockIdx.x * A.nb;
+  const int own = (int)(min(n0 + A.nb, A.n) - n0);
+  // lanes in turn: the m-th bond of a lane is word (warp * M + m) * 32 + lane, so
+  // that a warp's reads are consecutive
+  float *s_p = reinterpret_cast<float *>(s_bond + (size_t)NW * 32 * A.warps * A.bonds_per_lane);
+  const int nh = A.nh[blockIdx.x];
+  const int *halo = A.halo + (int64_t)blockIdx.x * kResHalo;
+  for (int k = threadIdx.x; k < DIM * (A.nb + nh); k += kResThreads) s_p[k] = 0.f;
+  // L lanes per node, the first of them its owner
+  const int L = A.lanes, tpw = 32 / L, lane = threadIdx.x & 31;
+  const int t = (threadIdx.x >> 5) * tpw + lane / L, l = lane % L;
+  const bool team = lane < tpw * L && t < own;
+  const bool lead = team && l == 0;
+  const int64_t i = n0 + t;
+  float x[DIM] = {}, r[DIM] = {}, z[DIM] = {}, dg[NB] = {}, mi[NB] = {};
+  bool fixed[DIM] = {};
+  int nk = 0;
+  float4 *bonds = s_bond + NW * ((size_t)(threadIdx.x >> 5) * A.bonds_per_lane * 32 + lane);
+  if (team) {
+    const int64_t r0 = A.rowptr[i] + l, r1 = A.rowptr[i + 1];
+    for (int64_t q = r0; q < r1; q += L, nk++) {
+      const double *b = A.blk + NB * q;
+      const float id = __int_as_float(A.lid[q]);
+      bonds[NW * 32 * nk] = make_float4((float)b[0], (float)b[1], (float)b[2],
+                                        DIM == 2 ? id : (float)b[3]);
+      if (DIM == 3) bonds[NW * 32 * nk + 1] = make_float4((float)b[4], (float)b[5], id, 0.f);
+    }
+  }
+  if (lead) {
+    const uint8_t fl = A.flags[i];
+    double b[NB];
+    for (int c = 0; c < NB; c++) {
+      b[c] = A.dblk[NB * i + c];
+      dg[c] = (float)b[c];
+    }
+    inv_diag32<DIM>(b, fl, mi);
+    for (int c = 0; c < DIM; c++) {
+      fixed[c] = fl >> c & 1;
+      r[c] = (float)A.rhs[DIM * i + c];
+    }
+  }
+  const float target = (float)(A.tol2 * *A.rr0);
+  df rz{0.f, 0.f};
+  float rr = (float)*A.rr0;
   float beta = 0.f;
   int it = 0;
-  bool ok = true;
-  while (it < max_iters) {
-    const float *pold = (it & 1) ? p0 : p1;
-    float *pnew = (it & 1) ? p1 : p0;
-    // phase 1: p_k = z_k + beta p_{k-1}, Ap_k, partials of p_k.Ap_k
-    float dot = 0.f;
-    const int64_t work = n * kG;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < work;
-         base += (int64_t)G * blockDim.x) {
-      const int64_t t = base + threadIdx.x;
-      const int64_t i = t / kG;
-      const int g = (int)(t % kG);
-      float acc[3] = {0.f, 0.f, 0.f}, tv[3];
-      if (i < n) {
-        const int64_t q1 = rowptr[i + 1];
-        for (int64_t qb = rowptr[i] + g; qb < q1; qb += 4 * kG) {
-          int jj[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) jj[u] = qb + u * kG < q1 ? cols[qb + u * kG] : -1;
-          float bb[4][NP], pj[4][3];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int j = jj[u] < 0 ? (int)i : jj[u];
-            const int64_t q = jj[u] < 0 ? qb : qb + u * kG;
-            const float4 *bp = reinterpret_cast<const float4 *>(blk + NP * q);
-            const float4 b0 = bp[0];
-            bb[u][0] = b0.x; bb[u][1] = b0.y; bb[u][2] = b0.z; bb[u][3] = b0.w;
-            if (DIM == 3) {
-              const float4 b1 = bp[1];
-              bb[u][4] = b1.x; bb[u][5] = b1.y; bb[u][6] = b1.z; bb[u][7] = b1.w;
-            }
-            for (int c = 0; c < DIM; c++) pj[u][c] = fmaf(beta, pold[DIM * j + c], z[DIM * j + c]);
-            if (DIM == 2) pj[u][2] = 0.f;
-          }
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (jj[u] < 0) continue;
-            sym_mul<float>(DIM, bb[u], pj[u], tv);
-            for (int c = 0; c < DIM; c++) acc[c] -= tv[c];
-          }
-        }
-      }
-      for (int o = kG / 2; o > 0; o >>= 1)
-        for (int c = 0; c < DIM; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-      if (i < n && g == 0) {
-        const uint8_t fl = flags[i];
-        float pi[3] = {0.f, 0.f, 0.f};
-        for (int c = 0; c < DIM; c++) {
-          pi[c] = fmaf(beta, pold[DIM * i + c], z[DIM * i + c]);
-          pnew[DIM * i + c] = pi[c];
-        }
-        sym_mul<float>(DIM, dblk + NB * i, pi, tv);
-        for (int c = 0; c < DIM; c++) {
-          const float yc = (fl >> c & 1) ? 0.f : acc[c] + tv[c];
-          ap[DIM * i + c] = yc;
-          dot = fmaf(pi[c], yc, dot);
-        }
+  uint32_t epoch = A.epoch + 1, arrivals = 0;
+  const uint32_t all = (uint32_t)(A.blocks + A.extra);
+  if (threadIdx.x == 0) s_stop = 0;
+  // z = M^-1 r, published with r.z and r.r; beta and the decision to go on
+  auto precondition = [&]() {
+    float v[2] = {0.f, 0.f};
+    if (lead) {
+      sym_mul<float>(DIM, mi, r, z);
+      for (int c = 0; c < DIM; c++) {
+        A.z[DIM * i + c] = z[c];
+        v[0] = fmaf(r[c], z[c], v[0]);
+        v[1] = fmaf(r[c], r[c], v[1]);
       }
     }
-    block_sum_f(dot, pap_p);
-    if (!(ok = coop_barrier(coop, expect, wait_ns))) break;
-    const double pap = coop_sum(pap_p, G);
-    const float alpha = (float)(pap != 0. ? rz / pap : 0.);
-    // phase 2: x += alpha p, r -= alpha Ap, z = block-Jacobi(r), partials of
-    // r.z and r.r
-    float drz = 0.f, drr = 0.f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)G * blockDim.x) {
-      const uint8_t fl = flags[i];
-      float rv[3] = {0.f, 0.f, 0.f}, zv[3] = {0.f, 0.f, 0.f};
-      for (int c = 0; c < DIM; c++) {
-        const int64_t k = DIM * i + c;
-        x[k] = fmaf(alpha, pnew[k], x[k]);
-        const float rk = fmaf(-alpha, ap[k], r[k]);
-        r[k] = rk;
-        drr = fmaf(rk, rk, drr);
-        rv[c] = (fl >> c & 1) ? 0.f : rk;
+    res_block_sum<2>(v, s_red);
+    if (threadIdx.x < 32) {
+      df s[2];
+      const bool ok = res_sum<2, true>(A, 1, epoch, arrivals += all, v, s);
+      if (it > 0) rr = s[1].hi;
+      if (threadIdx.x == 0) {
+        s_scal = it > 0 && rz.hi != 0.f ? df_div(s[0], rz) : 0.f;
+        s_stop = !ok ? 2 : !(rr > target) || it >= A.max_iters ? 1 : 0;
       }
-      block_jacobi<DIM, float>(dblk + NB * i, fl, rv, zv);
-      for (int c = 0; c < DIM; c++) {
-        z[DIM * i + c] = zv[c];
-        drz = fmaf(rv[c], zv[c], drz);
+      rz = s[0];
+    }
+    __syncthreads();
+    beta = s_scal;
+  };
+  precondition();
+  while (s_stop == 0) {
+    epoch++;
+    float p[DIM];
+    if (lead)
+      for (int c = 0; c < DIM; c++)
+        s_p[DIM * t + c] = p[c] = fmaf(beta, s_p[DIM * t + c], z[c]);
+    for (int h = threadIdx.x; h < nh; h += kResThreads) {
+      const int64_t g = halo[h];
+      float *ph = s_p + DIM * (A.nb + h);
+      if (DIM == 2) {
+        const float2 zz = __ldcg(reinterpret_cast<const float2 *>(A.z) + g);
+        ph[0] = fmaf(beta, ph[0], zz.x);
+        ph[1] = fmaf(beta, ph[1], zz.y);
+      } else {
+        for (int c = 0; c < DIM; c++) ph[c] = fmaf(beta, ph[c], __ldcg(A.z + DIM * g + c));
       }
     }
-    block_sum2_f(drz, drr, rz_p, rr_p);
-    if (!(ok = coop_barrier(coop, expect, wait_ns))) break;
-    const double rz_next = coop_sum(rz_p, G);
-    rr = coop_sum(rr_p, G);
-    beta = (float)(rz != 0. ? rz_next / rz : 0.);
-    rz = rz_next;
+    __syncthreads();
+    float acc[DIM] = {}, tv[DIM], ap[DIM] = {};
+#pragma unroll 2
+    for (int k = 0; k < nk; k++) {
+      const float4 w = bonds[NW * 32 * k];
+      if (DIM == 2) {
+        const float2 pj = reinterpret_cast<const float2 *>(s_p)[__float_as_int(w.w)];
+        acc[0] -= fmaf(w.x, pj.x, w.y * pj.y);
+        acc[1] -= fmaf(w.y, pj.x, w.z * pj.y);
+      } else {
+        const float4 w1 = bonds[NW * 32 * k + 1];
+        const float a[6] = {w.x, w.y, w.z, w.w, w1.x, w1.y};
+        sym_mul<float>(DIM, a, s_p + DIM * __float_as_int(w1.z), tv);
+        for (int c = 0; c < DIM; c++) acc[c] -= tv[c];
+      }
+    }
+    for (int c = 0; c < DIM; c++) {
+      const float mine = acc[c];
+      for (int o = 1; o < L; o++) acc[c] += __shfl_down_sync(0xffffffffu, mine, o);
+    }
+    float dot[1] = {0.f};
+    if (lead) {
+      sym_mul<float>(DIM, dg, p, tv);
+      for (int c = 0; c < DIM; c++) {
+        ap[c] = fixed[c] ? 0.f : acc[c] + tv[c];
+        dot[0] = fmaf(p[c], ap[c], dot[0]);
+      }
+    }
+    res_block_sum<1>(dot, s_red);
+    if (threadIdx.x < 32) {
+      df s[1];
+      const bool ok = res_sum<1, false>(A, 0, epoch, arrivals += all, dot, s);
+      if (threadIdx.x == 0) {
+        s_scal = s[0].hi != 0.f ? df_div(rz, s[0]) : 0.f;
+        if (!ok) s_stop = 2;
+      }
+    }
+    __syncthreads();
+    if (s_stop) break;
+    const float alpha = s_scal;
     it++;
-    if (!(rr > target)) break;
-    // the partials are rewritten next iteration only after the next barrier,
-    // which every block reaches after reading them
+    if (lead)
+      for (int c = 0; c < DIM; c++) {
+        x[c] = fmaf(alpha, p[c], x[c]);
+        r[c] = fmaf(-alpha, ap[c], r[c]);
+      }
+    precondition();
   }
+  if (lead)
+    for (int c = 0; c < DIM; c++) A.dx[DIM * i + c] = (double)x[c];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    res[0] = (double)it;
-    res[1] = rr;
+    A.res[0] = (double)it;
+    A.res[1] = (double)rr;
+    A.res[2] = (double)target;
   }
-  (void)ok;
 }
 
 __global__ void k_cg32_seed(float *fs, float *pold, int64_t m) {
@@ -989,10 +1155,13 @@ static cudaError_t qs_cg32(const StepParams &P, const DevPtrs &D, const QSWork &
   k_to_f32<<<qblk(m), 256, 0, s>>>(m, rhs, W.r32);
   if ((e = cudaMemsetAsync(W.x32, 0, sizeof(float) * m, s))) return e;
   // z_0 = M^-1 r_0 and rz_0; beta_{-1} = 0, p_{-1} = 0
-  if (dim == 2)
-    k_qs_precond32<2><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk32, W.r32, W.z32, rz_p);
-  else
-    k_qs_precond32<3><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk32, W.r32, W.z32, rz_p);
+  if (dim == 2) {
+    k_inv_diag32<2><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk, W.minv32);
+    k_qs_precond32<2><<<gn, 256, 0, s>>>(P.n, W.minv32, W.r32, W.z32, rz_p);
+  } else {
+    k_inv_diag32<3><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk, W.minv32);
+    k_qs_precond32<3><<<gn, 256, 0, s>>>(P.n, W.minv32, W.r32, W.z32, rz_p);
+  }
   k_qs_sum<<<1, 256, 0, s>>>(rz_p, gn, tot + 0);
   k_cg32_seed<<<qblk(m), 256, 0, s>>>(fs, pbuf[1], m);
   double rr0 = 0.;
@@ -1005,45 +1174,6 @@ static cudaError_t qs_cg32(const StepParams &P, const DevPtrs &D, const QSWork &
     *iters = 0;
     return cudaMemsetAsync(dx, 0, sizeof(double) * m, s);
   }
-  if (W.coop && W.coop_blocks > 0) {
-    // the whole solve in one cooperative launch
-    if ((e = cudaMemsetAsync(W.coop, 0, sizeof(unsigned), s))) return e;  // arrivals
-    if ((e = cudaMemsetAsync(W.coop + 2, 0, sizeof(unsigned), s))) return e;  // status
-    int64_t n = P.n;
-    const uint8_t *flags = D.flags;
-    const int64_t *rowptr = D.rowptr;
-    const int *cols = D.cols;
-    const float *blk = W.blk32, *dblk = W.dblk32;
-    float *p0 = pbuf[0], *p1 = pbuf[1], *ap = W.ap32, *x = W.x32, *r = W.r32, *z = W.z32;
-    double *part = W.cgpart;
-    const double *rz0 = tot + 0;
-    double tgt = target;
-    int mi = max_iters;
-    unsigned *coop = W.coop;
-    unsigned expect = (unsigned)W.coop_blocks + (unsigned)W.coop_extra;
-    uint64_t wait_ns = W.coop_wait_ns;
-    double *res = W.cgs + 6;
-    void *args[] = {&n, &flags, &rowptr, &cols, &blk, &dblk, &p0, &p1, &ap, &x, &r, &z,
-                    &part, &rz0, &tgt, &mi, &coop, &expect, &wait_ns, &res};
-    // p_{-1} = 0 lives in pbuf[1] (zeroed by the seed), p_0 goes to pbuf[0]
-    e = dim == 2 ? cudaLaunchCooperativeKernel((const void *)k_cg32_coop<2>, W.coop_blocks,
-                                               kCoopThreads, args, 0, s)
-                 : cudaLaunchCooperativeKernel((const void *)k_cg32_coop<3>, W.coop_blocks,
-                                               kCoopThreads, args, 0, s);
-    if (e != cudaSuccess) return e;
-    double hres[2] = {0., 0.};
-    int status = 0;
-    if ((e = cudaMemcpyAsync(hres, res, sizeof(hres), cudaMemcpyDeviceToHost, s))) return e;
-    if ((e = cudaMemcpyAsync(&status, W.coop + 2, sizeof(int), cudaMemcpyDeviceToHost, s)))
-      return e;
-    if ((e = cudaStreamSynchronize(s))) return e;
-    if (status != 0) return cudaErrorTimeout;
-    it = (int)hres[0];
-    *converged = !(hres[1] > target) || it < max_iters;
-    k_to_f64<<<qblk(m), 256, 0, s>>>(m, W.x32, dx);
-    *iters = it;
-    return cudaGetLastError();
-  }
   while (it < max_iters) {
     for (int q = 0; q < check_every && it < max_iters; q++, it++) {
       const int cur = it & 1, prv = cur ^ 1;
@@ -1051,14 +1181,14 @@ static cudaError_t qs_cg32(const StepParams &P, const DevPtrs &D, const QSWork &
         k_cg32_dir_spmv<2><<<gg, 256, 0, s>>>(P.n, D.flags, D.rowptr, D.cols, W.blk32,
                                               W.dblk32, W.z32, pbuf[prv], pbuf[cur], W.ap32,
                                               tot + cur, pap_p, W.ticket, tot + 2, fs);
-        k_cg32_update<2><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk32, pbuf[cur], W.ap32, W.x32,
+        k_cg32_update<2><<<gn, 256, 0, s>>>(P.n, W.minv32, pbuf[cur], W.ap32, W.x32,
                                             W.r32, W.z32, tot + cur, rz_p, rr_p, W.ticket + 1,
                                             tot + prv, tot + 3, fs);
       } else {
         k_cg32_dir_spmv<3><<<gg, 256, 0, s>>>(P.n, D.flags, D.rowptr, D.cols, W.blk32,
                                               W.dblk32, W.z32, pbuf[prv], pbuf[cur], W.ap32,
                                               tot + cur, pap_p, W.ticket, tot + 2, fs);
-        k_cg32_update<3><<<gn, 256, 0, s>>>(P.n, D.flags, W.dblk32, pbuf[cur], W.ap32, W.x32,
+        k_cg32_update<3><<<gn, 256, 0, s>>>(P.n, W.minv32, pbuf[cur], W.ap32, W.x32,
                                             W.r32, W.z32, tot + cur, rz_p, rr_p, W.ticket + 1,
                                             tot + prv, tot + 3, fs);
       }
@@ -1075,25 +1205,137 @@ static cudaError_t qs_cg32(const StepParams &P, const DevPtrs &D, const QSWork &
   return cudaGetLastError();
 }
 
-// Blocks of the cooperative solve: up to four blocks of kCoopThreads per SM
-// that can be resident together, at most one per kCoopThreads (node, lane)
-// items; 0 if the device cannot launch it cooperatively.  (One block of 1024
-// threads per SM, fewer arrivals per barrier, measured slower.)
-int qs_coop_blocks(int64_t n, int dim) {
-  int dev = 0, sms = 0, coop = 0, per = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+// The whole FP32 solve in one cooperative launch; *status = NLM_ERR_TIMEOUT
+// when a wait ran out (dx is then undefined).
+static cudaError_t qs_cg32_res(const StepParams &P, const DevPtrs &D, QSWork &W,
+                               const double *rhs, double *dx, double tol, int max_iters,
+                               int *iters, bool *converged, int *status, cudaStream_t s) {
+  cudaError_t e = qs_dot(rhs, rhs, (int64_t)P.dim * P.n, W.part, W.sc + 3, s);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(W.kr.status, 0, 2 * sizeof(int), s);  // and the count
+  if (e != cudaSuccess) return e;
+  // iteration numbers go on from solve to solve, so no word holds one that a
+  // later solve waits for
+  if (W.epoch > 0xffffffffu - (uint32_t)max_iters - 4) {
+    e = cudaMemsetAsync(W.kr.words, 0, sizeof(uint64_t) * 3 * W.kr.stride, s);
+    if (e != cudaSuccess) return e;
+    W.epoch = 0;
+  }
+  CgRes A = W.kr;
+  A.epoch = W.epoch;
+  W.epoch += (uint32_t)max_iters + 2;
+  A.rhs = rhs;
+  A.dx = dx;
+  A.rr0 = W.sc + 3;
+  A.tol2 = tol * tol;
+  A.max_iters = max_iters;
+  void *args[] = {&A};
+  e = cudaLaunchCooperativeKernel(
+      P.dim == 2 ? (const void *)k_cg32_res<2> : (const void *)k_cg32_res<3>, A.blocks,
+      kResThreads, args, W.res_smem, s);
+  double r[4] = {};
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(r, A.res, sizeof(r), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(status, A.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return e;
+  *iters = (int)r[0];
+  *converged = !(r[1] > r[2]) || *iters < max_iters;
+  return cudaSuccess;
+}
+
+// Layout of the resident solve: blocks, node ranges, lanes per node, halo
+// lists.  blocks = 0 where it does not apply: no cooperative launch, or a
+// block's tangent (16 bytes per 2-D bond, 32 per 3-D one) or halo that does
+// not fit its SM -- above about 1.8 million 2-D bonds the tangent streams from
+// L2 in the two-launch form.
+cudaError_t qs_res_setup(const StepParams &P, const DevPtrs &D, const int64_t *rowptr_host,
+                         QSWork &W, const std::function<cudaError_t(void **, size_t)> &alloc,
+                         cudaStream_t s) {
+  CgRes &A = W.kr;
+  A.blocks = 0;
+  int dev = 0, sms = 0, coop = 0, smem = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (!coop || sms <= 0) return 0;
-  cudaError_t e =
-      dim == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg32_coop<2>, kCoopThreads, 0)
-               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg32_coop<3>, kCoopThreads, 0);
-  if (e != cudaSuccess || per <= 0) {
-    cudaGetLastError();
-    return 0;
+  cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (!coop || sms <= 0 || P.n == 0) return cudaSuccess;
+  const int64_t n = P.n;
+  int64_t longest = 0;
+  for (int64_t k = 0; k < n; k++)
+    longest = std::max(longest, rowptr_host[k + 1] - rowptr_host[k]);
+  // at least 64 nodes per block (fewer words to add), unless their tangent
+  // does not fit
+  int nb = 0, blocks = 0, L = 0, warps = 0, M = 0;
+  size_t words = 0;
+  smem -= 1024;  // the kernel's static arrays
+  for (int64_t most : {(n + 63) / 64, n}) {
+    const int64_t want = std::min<int64_t>(sms, most);
+    nb = (int)std::min<int64_t>((n + want - 1) / want, 1 << 20);
+    blocks = (int)((n + nb - 1) / nb);
+    L = 8;
+    while (L > 1 && 32 / L * (kResThreads / 32) < nb) L--;
+    warps = (nb + 32 / L - 1) / (32 / L);
+    M = (int)((longest + L - 1) / L);
+    words = (size_t)(P.dim == 2 ? 16 : 32) * 32 * warps * M;
+    if (nb <= kResThreads && words <= (size_t)smem) break;
   }
-  const int64_t need = std::max<int64_t>(1, (n * kG + kCoopThreads - 1) / kCoopThreads);
-  return (int)std::min<int64_t>((int64_t)sms * std::min(per, 4), need);
+  if (nb > kResThreads || words > (size_t)smem) return cudaSuccess;
+  const int64_t nnz = rowptr_host[n];
+  void *p[6] = {};
+  const size_t bytes[6] = {sizeof(int) * (size_t)blocks * kResHalo, sizeof(int) * (size_t)blocks,
+                           sizeof(uint16_t) * (size_t)(nnz + 1),
+                           sizeof(uint64_t) * (3 * (size_t)blocks + 1),
+                           sizeof(float) * (size_t)P.dim * n, sizeof(double) * 4};
+  for (int k = 0; k < 6; k++)
+    if ((e = alloc(&p[k], bytes[k])) != cudaSuccess) return e;
+  std::vector<int> nh(blocks);
+  k_cg_res_setup<<<blocks, kResThreads, 0, s>>>(n, nb, D.rowptr, D.cols, (int *)p[0], (int *)p[1],
+                                                (uint16_t *)p[2]);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(nh.data(), p[1], bytes[1], cudaMemcpyDeviceToHost, s))) return e;
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+  int hmax = 0;
+  for (int v : nh) {
+    if (v < 0) return cudaSuccess;
+    hmax = std::max(hmax, v);
+  }
+  W.res_smem = words + sizeof(float) * P.dim * (size_t)(nb + hmax);
+  const void *kern = P.dim == 2 ? (const void *)k_cg32_res<2> : (const void *)k_cg32_res<3>;
+  int per = 0;
+  if (W.res_smem > (size_t)smem ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kResThreads, W.res_smem) !=
+          cudaSuccess ||
+      per < 1) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  A.n = n;
+  A.nb = nb;
+  A.lanes = L;
+  A.warps = warps;
+  A.bonds_per_lane = M;
+  A.flags = D.flags;
+  A.rowptr = D.rowptr;
+  A.halo = (const int *)p[0];
+  A.nh = (const int *)p[1];
+  A.lid = (const uint16_t *)p[2];
+  A.words = (unsigned long long *)p[3];
+  A.stride = blocks;
+  A.status = (int *)(A.words + 3 * (size_t)blocks);
+  A.count = (unsigned *)A.status + 1;
+  if ((e = cudaMemsetAsync(p[3], 0, bytes[3], s)) != cudaSuccess) return e;
+  W.epoch = 0;
+  A.z = (float *)p[4];
+  A.res = (double *)p[5];
+  A.blk = W.blk;
+  A.dblk = W.dblk;
+  A.blocks = blocks;
+  return cudaSuccess;
 }
 
 // Newton correction (-K) dx = rhs.  The FP32 solve is tried first; when it
@@ -1103,14 +1345,24 @@ int qs_coop_blocks(int64_t n, int dim) {
 // FP64 for the rest of the load step.
 constexpr int kCg32Cap = 800;
 
-cudaError_t qs_cg(const StepParams &P, const DevPtrs &D, const QSWork &W, const double *rhs,
+cudaError_t qs_cg(const StepParams &P, const DevPtrs &D, QSWork &W, const double *rhs,
                   double *dx, double tol, int max_iters, int check_every, int *iters,
                   bool *use64, cudaStream_t s) {
   int it32 = 0;
   if (!*use64) {
     bool conv = false;
-    cudaError_t e = qs_cg32(P, D, W, rhs, dx, tol, std::min(max_iters, kCg32Cap), check_every,
-                            &it32, &conv, s);
+    cudaError_t e = cudaSuccess;
+    int status = 0;
+    const int cap = std::min(max_iters, kCg32Cap);
+    if (W.kr.blocks > 0) {
+      e = qs_cg32_res(P, D, W, rhs, dx, tol, cap, &it32, &conv, &status, s);
+      if (e == cudaSuccess && status != 0) {
+        if (W.res_only) return cudaErrorTimeout;
+        W.kr.blocks = 0;  // the two-launch form from now on
+      }
+    }
+    if (e == cudaSuccess && (W.kr.blocks == 0 || status != 0))
+      e = qs_cg32(P, D, W, rhs, dx, tol, cap, check_every, &it32, &conv, s);
     if (e != cudaSuccess || conv || max_iters <= kCg32Cap) {
       *iters = it32;
       return e;

@@ -147,22 +147,21 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
     if (e == cudaSuccess) e = q->alloc(p, m);
   if (e == cudaSuccess) e = q->alloc(&q->W.blk32, (size_t)(NB == 3 ? 4 : 8) * (nnz + 1));
   if (e == cudaSuccess) e = q->alloc(&q->W.dblk32, (size_t)NB * n);
+  if (e == cudaSuccess) e = q->alloc(&q->W.minv32, (size_t)NB * n);
   q->W.nnz = nnz;
   if (e == cudaSuccess) e = q->alloc(&q->W.ticket, 4);
   if (e == cudaSuccess) e = cudaMemset(q->W.ticket, 0, 4 * sizeof(unsigned));
-  if (e == cudaSuccess && prm->krylov_launch == 1) {
-    q->W.coop_blocks = qs_coop_blocks(n, h->dim);
-    if (q->W.coop_blocks > 0) {
-      e = q->alloc(&q->W.coop, 4);
-      if (e == cudaSuccess) e = cudaMemset(q->W.coop, 0, 4 * sizeof(unsigned));
-      q->W.coop_extra = std::max(0, prm->barrier_extra);
-      const double lim = prm->wait_limit_s > 0. ? prm->wait_limit_s : 1.0;
-      q->W.coop_wait_ns = (uint64_t)(std::min(lim, 60.0) * 1e9);
-    }
-  }
   if (e == cudaSuccess) e = q->alloc(&q->W.sc, 8);
   if (e == cudaSuccess) e = q->alloc(&q->W.blk, (size_t)NB * (nnz + 1));
   if (e == cudaSuccess) e = q->alloc(&q->W.dblk, (size_t)NB * n);
+  if (e == cudaSuccess)
+    e = qs_res_setup(h->P, h->D, h->rowptr.data(), q->W,
+                     [&](void **p, size_t bytes) { return q->alloc((char **)p, bytes); },
+                     h->stream);
+  q->W.res_only = prm->krylov_launch == 1;
+  q->W.kr.extra = std::max(0, std::min(prm->barrier_extra, 64));
+  q->W.kr.wait_ns =
+      (uint64_t)(std::min(prm->wait_limit_s > 0. ? prm->wait_limit_s : 1.0, 60.0) * 1e9);
   if (e == cudaSuccess) e = q->alloc(&q->count, 1);
   if (e == cudaSuccess) e = q->alloc(&q->saved, (size_t)h->S * n);
   if (e == cudaSuccess) e = q->alloc(&q->cand, (size_t)h->S * n);

@@ -1,9 +1,36 @@
 // qs_internal.h -- work buffers and launchers of the quasi-static solver.
 #pragma once
 
+#include <functional>
+
 #include "fd_internal.h"
 
 namespace nlm {
+
+// The FP32 Krylov solve in one cooperative launch (qs.cu: k_cg32_res).
+constexpr int kResHalo = 2048;  // most halo nodes of a block
+struct CgRes {
+  int64_t n;
+  int blocks, nb;          // grid, consecutive nodes of a block
+  int lanes, warps, bonds_per_lane;  // lanes per node, warps with nodes, longest share
+  uint32_t epoch;          // iteration numbers of this solve start above it
+  const uint8_t *flags;
+  const int64_t *rowptr;
+  const int *halo, *nh;    // kResHalo ids per block, and how many
+  const uint16_t *lid;     // per bond: local id of the neighbour
+  const double *blk, *dblk, *rhs;
+  double *dx;
+  float *z;                // DIM per node
+  unsigned long long *words;  // 3 x stride: (iteration, FP32 partial) of each block
+  int stride, extra;       // extra: arrivals a sum waits for that nobody makes (tests)
+  unsigned *count;         // arrivals of this solve
+  const double *rr0;       // r.r of the right-hand side
+  double tol2;
+  int max_iters;
+  int *status;
+  uint64_t wait_ns;        // bound of each wait
+  double *res;
+};
 
 struct QSWork {
   double *res;    // residual, DIM per node
@@ -19,20 +46,18 @@ struct QSWork {
   double *dblk;   // diagonal blocks per node
   double *res0;   // force at the previous converged state
   // FP32 Krylov solve: tangent copies and CG vectors
-  float *blk32, *dblk32, *r32, *z32, *p32, *p32b, *ap32, *x32;
+  float *blk32, *dblk32, *minv32, *r32, *z32, *p32, *p32b, *ap32, *x32;
   int64_t nnz;
-  // the FP32 solve in one cooperative launch (coop == null: two launches
-  // per iteration): barrier words (arrivals, generation, status), grid
-  // size, extra arrivals a barrier waits for (testing the bound only) and
-  // the bound of each barrier wait
-  unsigned *coop;
-  int coop_blocks;
-  int coop_extra;
-  uint64_t coop_wait_ns;
+  CgRes kr;         // kr.blocks == 0: two launches per iteration
+  size_t res_smem;
+  uint32_t epoch;   // iteration numbers used up by earlier solves
+  bool res_only;    // a wait that runs out is an error (else: two launches)
 };
 
-// Grid size of the cooperative FP32 solve for n nodes (0: not available).
-int qs_coop_blocks(int64_t n, int dim);
+// Lay out the resident FP32 solve in W.kr (blocks = 0: not available).
+cudaError_t qs_res_setup(const StepParams &P, const DevPtrs &D, const int64_t *rowptr_host,
+                         QSWork &W, const std::function<cudaError_t(void **, size_t)> &alloc,
+                         cudaStream_t s);
 
 // count != NULL: bonds past the critical strain break during the evaluation
 // (RNPBond::getBondEF) and the number broken is added to *count.
@@ -42,7 +67,7 @@ cudaError_t qs_residual(const StepParams &P, const DevPtrs &D, const double *u, 
 cudaError_t qs_dot(const double *a, const double *b, int64_t m, double *part, double *out,
                    cudaStream_t s);
 // use64: in/out, FP64 Krylov solve (set when the FP32 solve did not converge)
-cudaError_t qs_cg(const StepParams &P, const DevPtrs &D, const QSWork &W, const double *rhs,
+cudaError_t qs_cg(const StepParams &P, const DevPtrs &D, QSWork &W, const double *rhs,
                   double *dx, double tol, int max_iters, int check_every, int *iters,
                   bool *use64, cudaStream_t s);
 // Entries per partial-sum array of the CG (4 arrays live in QSWork::cgpart).

@@ -39,7 +39,8 @@ struct nlm_batch {
   bool tile_ok = false;  // tile store over the combined layout (2-D)
   int *bc_nodes = nullptr;
   int64_t n_bc_nodes = 0;
-  double *stage = nullptr;
+  double *stage = nullptr;    // up to three fields of one specimen, caller's layout
+  int *perm_dev = nullptr;    // internal -> original node id, per specimen at its offset
   // graphs
   int graph_steps = 0;
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
@@ -560,7 +561,10 @@ int nlm_batch_create(const nlm_fd_desc *descs, int nspec, nlm_batch **out) {
   BTRY(b->alloc(&D.v32[0], (size_t)(S / 2) * N));
   BTRY(b->alloc(&D.v32[1], (size_t)(S / 2) * N));
   BTRY(b->alloc(&D.f32, (size_t)S * N));
-  BTRY(b->alloc(&b->stage, 3 * (size_t)N));
+  int64_t nmax = 0;
+  for (int s = 0; s < nspec; s++) nmax = std::max<int64_t>(nmax, descs[s].n_nodes);
+  BTRY(b->alloc(&b->stage, 9 * (size_t)nmax));
+  BTRY(b->alloc(&b->perm_dev, (size_t)N));
   double *fx;
   BTRY(b->alloc(&fx, (size_t)S * N));
   D.fext = fx;
@@ -569,11 +573,9 @@ int nlm_batch_create(const nlm_fd_desc *descs, int nspec, nlm_batch **out) {
   BTRY(cudaMemsetAsync(D.f32, 0, sizeof(float) * S * N, st));
   BTRY(cudaMemsetAsync(fx, 0, sizeof(double) * S * N, st));
   // initial states
-  int *dperm;
-  BTRY(b->alloc(&dperm, N));
   for (int s = 0; s < nspec; s++) {
     const nlm_fd_desc &d = descs[s];
-    if (!d.u0 && !d.v0) continue;
+    int *dperm = b->perm_dev + b->off[s];
     BTRY(cudaMemcpyAsync(dperm, b->perm[s].data(), sizeof(int) * d.n_nodes, cudaMemcpyHostToDevice, st));
     const unsigned g = nblk(d.n_nodes, 256);
     if (d.u0) {
@@ -700,28 +702,21 @@ int nlm_batch_get_state(nlm_batch *b, int s, double *u, double *v, double *f) {
   const int64_t n = b->n[s], off = b->off[s];
   const int S = b->S;
   cudaStream_t st = b->stream;
-  int *dperm = nullptr;
-  NLM_CUDA(cudaMalloc(&dperm, sizeof(int) * (n + 1)));
-  cudaError_t e = cudaMemcpyAsync(dperm, b->perm[s].data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
+  const int *perm = b->perm_dev + off;
   const unsigned g = nblk(n, 256);
   const int vi = b->scheme == NLM_CENTRAL_DIFFERENCE ? b->cur : 0;
-  if (e == cudaSuccess && u) {
-    k_gather_split<<<g, 256, 0, st>>>(n, S, dperm, b->D.u32[b->cur] + (S / 2) * off, b->stage);
-    e = cudaMemcpyAsync(u, b->stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  if (e == cudaSuccess && v) {
-    k_gather_split<<<g, 256, 0, st>>>(n, S, dperm, b->D.v32[vi] + (S / 2) * off, b->stage);
-    e = cudaMemcpyAsync(v, b->stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  if (e == cudaSuccess && f) {
-    k_gather_f32<<<g, 256, 0, st>>>(n, S, dperm, b->D.f32 + (size_t)S * off, b->stage);
-    e = cudaMemcpyAsync(f, b->stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  cudaStreamSynchronize(st);
-  cudaFree(dperm);
+  const size_t bytes = sizeof(double) * 3 * n;
+  double *su = b->stage, *sv = su + 3 * n, *sf = sv + 3 * n;
+  touch_pages({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
+  if (u) k_gather_split<<<g, 256, 0, st>>>(n, S, perm, b->D.u32[b->cur] + (S / 2) * off, su);
+  if (v) k_gather_split<<<g, 256, 0, st>>>(n, S, perm, b->D.v32[vi] + (S / 2) * off, sv);
+  if (f) k_gather_f32<<<g, 256, 0, st>>>(n, S, perm, b->D.f32 + (size_t)S * off, sf);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && u) e = cudaMemcpyAsync(u, su, bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && v) e = cudaMemcpyAsync(v, sv, bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && f) e = cudaMemcpyAsync(f, sf, bytes, cudaMemcpyDeviceToHost, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return cuda_fail(e, "batch state download");
   return NLM_OK;
 }

@@ -12,8 +12,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -32,6 +34,10 @@ void set_error(const std::string &msg);
 const char *last_error();
 int cuda_fail(cudaError_t e, const char *what);
 int fail(int code, const std::string &msg);
+
+// Make the pages of the caller's output arrays resident (null pointers are
+// skipped, contents stay).
+void touch_pages(std::initializer_list<std::pair<void *, size_t>> arrays);
 
 inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 

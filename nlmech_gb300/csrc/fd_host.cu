@@ -1161,6 +1161,8 @@ int get_state_impl(nlm_fd *h, double *u, double *v, double *f, bool keep_z) {
   // gather each requested field into its own staging slot, copy all out,
   // synchronise once
   double *su = h->stage, *sv = h->stage + 3 * n, *sf = h->stage + 6 * n;
+  const size_t bytes = sizeof(double) * 3 * n;
+  touch_pages({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
   if (u) {
     if (fp32)
       k_gather_split<<<g, 256, 0, s>>>(n, h->S, P, h->D.u32[h->cur], su, keep_z);

@@ -23,6 +23,40 @@ int fail(int code, const std::string &msg) {
 
 const char *last_error() { return g_err.c_str(); }
 
+// Pages of a fresh allocation that a device copy meets first are made resident
+// one fault at a time: three fresh arrays of 24 MB took 40 ms to receive (1.8
+// GB/s), the same arrays touched before 0.5 ms.  One write of the byte already
+// there per page, by up to four threads (1.2 ms for the 72 MB; 2.9 ms with one,
+// 3.9 ms with sixteen), makes them resident; arrays that were resident cost a
+// few microseconds.  Small arrays usually lie in memory the process has used.
+void touch_pages(std::initializer_list<std::pair<void *, size_t>> arrays) {
+  constexpr size_t kMin = 4 << 20, kPage = 4096;
+  size_t total = 0;
+  for (auto &a : arrays)
+    if (a.first) total += a.second;
+  if (total < kMin) return;
+  const unsigned nt = (unsigned)std::min<size_t>(4, total / kMin);
+  auto part = [&](unsigned w) {
+    for (auto &a : arrays) {
+      if (!a.first) continue;
+      volatile char *p = static_cast<volatile char *>(a.first);
+      const size_t seg = (a.second / kPage / nt + 1) * kPage;
+      for (size_t o = w * seg; o < std::min(a.second, (w + 1) * seg); o += kPage) p[o] = p[o];
+      if (w == nt - 1 && a.second) p[a.second - 1] = p[a.second - 1];
+    }
+  };
+  std::vector<std::thread> pool;
+  unsigned w = 1;
+  try {
+    pool.reserve(nt);
+    for (; w < nt; w++) pool.emplace_back(part, w);
+  } catch (...) {
+    for (unsigned q = w; q < nt; q++) part(q);  // no thread to be had
+  }
+  part(0);
+  for (auto &t : pool) t.join();
+}
+
 // ---- host restatement of the deck-level set-up --------------------------
 
 // Displacement_BC / Force_BC region membership (uLoading.cpp:93-160,

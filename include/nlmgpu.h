@@ -238,6 +238,14 @@ int nlm_set_device(int device);
 int nlm_neighbor_search(int dim, int64_t n, const double *x, double horizon,
                         int64_t *rowptr, int32_t *cols);
 
+/* The same search once for both outputs: create searches and gives the number
+ * of entries, get copies rowptr (n+1) and cols (nnz, may be NULL) out. */
+typedef struct nlm_neighbors nlm_neighbors;
+int nlm_neighbors_create(int dim, int64_t n, const double *x, double horizon, int64_t *nnz,
+                         nlm_neighbors **out);
+int nlm_neighbors_get(nlm_neighbors *h, int64_t *rowptr, int32_t *cols);
+int nlm_neighbors_destroy(nlm_neighbors *h);
+
 /* Same result as nlm_neighbor_search, with no device allocation.  No
  * counterpart in the reference (it allocates through its std::vector
  * neighbour lists); this entry serves callers that must not allocate device

@@ -707,7 +707,7 @@ int nlm_batch_get_state(nlm_batch *b, int s, double *u, double *v, double *f) {
   const int vi = b->scheme == NLM_CENTRAL_DIFFERENCE ? b->cur : 0;
   const size_t bytes = sizeof(double) * 3 * n;
   double *su = b->stage, *sv = su + 3 * n, *sf = sv + 3 * n;
-  touch_pages({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
+  prefault({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
   if (u) k_gather_split<<<g, 256, 0, st>>>(n, S, perm, b->D.u32[b->cur] + (S / 2) * off, su);
   if (v) k_gather_split<<<g, 256, 0, st>>>(n, S, perm, b->D.v32[vi] + (S / 2) * off, sv);
   if (f) k_gather_f32<<<g, 256, 0, st>>>(n, S, perm, b->D.f32 + (size_t)S * off, sf);

@@ -37,7 +37,7 @@ int fail(int code, const std::string &msg);
 
 // Make the pages of the caller's output arrays resident (null pointers are
 // skipped, contents stay).
-void touch_pages(std::initializer_list<std::pair<void *, size_t>> arrays);
+void prefault(std::initializer_list<std::pair<void *, size_t>> arrays);
 
 inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 

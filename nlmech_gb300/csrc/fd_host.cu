@@ -645,47 +645,68 @@ int nlm_set_device(int device) {
   return NLM_OK;
 }
 
-int nlm_neighbor_search(int dim, int64_t n, const double *x, double horizon, int64_t *rowptr,
-                        int32_t *cols) {
-  if (n < 0 || (n > 0 && !x) || !rowptr || dim < 1 || dim > 3 || !(horizon > 0.))
+struct nlm_neighbors {
+  NeighborSearch R;
+};
+
+namespace {
+int search_into(NeighborSearch &R, int dim, int64_t n, const double *x, double horizon,
+                bool want_cols) {
+  if (n < 0 || (n > 0 && !x) || dim < 1 || dim > 3 || !(horizon > 0.))
     return fail(NLM_ERR_INVALID, "nlm_neighbor_search: bad arguments");
   if (n > INT32_MAX - 1) return fail(NLM_ERR_INVALID, "too many nodes");
-  if (!finite_all(x, 3 * n)) return fail(NLM_ERR_NONFINITE, "non-finite coordinate");
-  cudaStream_t s;
-  NLM_CUDA(cudaStreamCreate(&s));
-  double *dx = nullptr;
-  NeighborBuild nb;
+  R.n = n;
+  if (n == 0) return NLM_OK;
   std::string why;
-  auto cleanup = [&]() {
-    cudaFree(dx); cudaFree(nb.perm); cudaFree(nb.pos); cudaFree(nb.rowptr); cudaFree(nb.cols);
-    cudaStreamDestroy(s);
-  };
-  cudaError_t e = cudaMalloc(&dx, sizeof(double) * 3 * (n + 1));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s);
-  const Grid g = make_grid(dim, n, x, horizon);
-  if (e == cudaSuccess) e = build_neighbors(nb, dim, n, dx, g, 4, s, why);
-  if (e != cudaSuccess) {
-    int rc = why.empty() ? cuda_fail(e, "neighbour search") : fail(NLM_ERR_INVALID, why);
-    cleanup();
+  const cudaError_t e = search_neighbors(R, n, x, horizon, want_cols, why);
+  if (e == cudaSuccess) return NLM_OK;
+  if (why.empty()) return cuda_fail(e, "neighbour search");
+  return fail(why[0] == 'n' ? NLM_ERR_NONFINITE : NLM_ERR_INVALID, why);
+}
+
+int search_out(NeighborSearch &R, int64_t *rowptr, int32_t *cols) {
+  rowptr[0] = 0;
+  if (R.n == 0) return NLM_OK;
+  prefault({{rowptr, sizeof(int64_t) * (R.n + 1)}, {cols, sizeof(int32_t) * R.nnz}});
+  NLM_CUDA(cudaMemcpyAsync(rowptr, R.rowptr, sizeof(int64_t) * (R.n + 1), cudaMemcpyDeviceToHost,
+                           R.s));
+  if (cols && R.nnz)
+    NLM_CUDA(cudaMemcpyAsync(cols, R.cols, sizeof(int32_t) * R.nnz, cudaMemcpyDeviceToHost, R.s));
+  NLM_CUDA(cudaStreamSynchronize(R.s));
+  return NLM_OK;
+}
+}  // namespace
+
+int nlm_neighbor_search(int dim, int64_t n, const double *x, double horizon, int64_t *rowptr,
+                        int32_t *cols) {
+  if (!rowptr) return fail(NLM_ERR_INVALID, "nlm_neighbor_search: bad arguments");
+  NeighborSearch R;
+  const int rc = search_into(R, dim, n, x, horizon, cols != nullptr);
+  return rc ? rc : search_out(R, rowptr, cols);
+}
+
+int nlm_neighbors_create(int dim, int64_t n, const double *x, double horizon, int64_t *nnz,
+                         nlm_neighbors **out) {
+  if (!nnz || !out) return fail(NLM_ERR_INVALID, "null argument");
+  *out = nullptr;
+  nlm_neighbors *h = new nlm_neighbors();
+  const int rc = search_into(h->R, dim, n, x, horizon, true);
+  if (rc) {
+    delete h;
     return rc;
   }
-  std::vector<int> perm(n);
-  std::vector<int64_t> rp(n + 1);
-  std::vector<int> cc(nb.nnz);
-  e = cudaMemcpy(perm.data(), nb.perm, sizeof(int) * n, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(rp.data(), nb.rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && nb.nnz) e = cudaMemcpy(cc.data(), nb.cols, sizeof(int) * nb.nnz, cudaMemcpyDeviceToHost);
-  cleanup();
-  if (e != cudaSuccess) return cuda_fail(e, "neighbour download");
-  std::vector<int64_t> inv(n);
-  for (int64_t i = 0; i < n; i++) inv[perm[i]] = i;
-  rowptr[0] = 0;
-  for (int64_t o = 0; o < n; o++) rowptr[o + 1] = rowptr[o] + (rp[inv[o] + 1] - rp[inv[o]]);
-  if (cols)
-    for (int64_t o = 0; o < n; o++) {
-      const int64_t s0 = rp[inv[o]], len = rp[inv[o] + 1] - s0;
-      for (int64_t k = 0; k < len; k++) cols[rowptr[o] + k] = perm[cc[s0 + k]];
-    }
+  *nnz = h->R.nnz;
+  *out = h;
+  return NLM_OK;
+}
+
+int nlm_neighbors_get(nlm_neighbors *h, int64_t *rowptr, int32_t *cols) {
+  if (!h || !rowptr) return fail(NLM_ERR_INVALID, "null argument");
+  return search_out(h->R, rowptr, cols);
+}
+
+int nlm_neighbors_destroy(nlm_neighbors *h) {
+  delete h;
   return NLM_OK;
 }
 
@@ -1162,7 +1183,7 @@ int get_state_impl(nlm_fd *h, double *u, double *v, double *f, bool keep_z) {
   // synchronise once
   double *su = h->stage, *sv = h->stage + 3 * n, *sf = h->stage + 6 * n;
   const size_t bytes = sizeof(double) * 3 * n;
-  touch_pages({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
+  prefault({{u, bytes}, {v, bytes}, {f, bytes}});  // while the steps run
   if (u) {
     if (fp32)
       k_gather_split<<<g, 256, 0, s>>>(n, h->S, P, h->D.u32[h->cur], su, keep_z);

@@ -24,6 +24,19 @@ struct NeighborBuild {  // device arrays, owned by the caller after the build
   int *cols = nullptr;        // sorted ids, rows ascending in original id
 };
 
+// Result of search_neighbors on the device: CSR in the caller's node ids.
+struct NeighborSearch {
+  int64_t n = 0, nnz = 0;
+  cudaStream_t s = nullptr;
+  void *arena = nullptr;
+  int64_t *rowptr = nullptr;  // in the arena
+  int *cols = nullptr;
+  ~NeighborSearch();
+};
+// n > 0; why is set where the failure is the input's.
+cudaError_t search_neighbors(NeighborSearch &R, int64_t n, const double *x, double horizon,
+                             bool want_cols, std::string &why);
+
 struct SellStore {
   int64_t nslices = 0, entries = 0;
   int maxw = 0;

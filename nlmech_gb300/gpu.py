@@ -63,13 +63,16 @@ def neighbor_search(x, horizon, dim=2):
     """GPU cell-list neighbour lists in original ids (rowptr int64, cols int32)."""
     x = np.ascontiguousarray(x, dtype=np.float64).reshape(-1, 3)
     n = x.shape[0]
-    rowptr = np.zeros(n + 1, dtype=np.int64)
     L = load()
-    _check(L.nlm_neighbor_search(C.c_int(dim), C.c_int64(n), abi.dptr(x), C.c_double(horizon),
-                                 abi.ptr(rowptr, C.c_int64), C.POINTER(C.c_int32)()))
-    cols = np.zeros(int(rowptr[-1]), dtype=np.int32)
-    _check(L.nlm_neighbor_search(C.c_int(dim), C.c_int64(n), abi.dptr(x), C.c_double(horizon),
-                                 abi.ptr(rowptr, C.c_int64), abi.ptr(cols, C.c_int32)))
+    h, nnz = C.c_void_p(), C.c_int64()
+    _check(L.nlm_neighbors_create(C.c_int(dim), C.c_int64(n), abi.dptr(x), C.c_double(horizon),
+                                  C.byref(nnz), C.byref(h)))
+    try:
+        rowptr = np.zeros(n + 1, dtype=np.int64)
+        cols = np.zeros(nnz.value, dtype=np.int32)
+        _check(L.nlm_neighbors_get(h, abi.ptr(rowptr, C.c_int64), abi.ptr(cols, C.c_int32)))
+    finally:
+        L.nlm_neighbors_destroy(h)
     return rowptr, cols
 
 

@@ -82,13 +82,13 @@ int batch_launch(nlm_batch *b, StepArgs a) {
   if (all_tile) {
     a.i0 = b->buckets.front().i0;
     a.i1 = b->buckets.back().i1;
-    cudaError_t e = launch_rnp_step_fp32(b->P, b->D, b->T, a, NLM_DECOMP_TILE_LOCAL, b->stream);
+    cudaError_t e = launch_rnp_step_fp32(b->P, b->D, a, NLM_DECOMP_TILE_LOCAL, b->stream);
     return e == cudaSuccess ? NLM_OK : cuda_fail(e, "batched step launch");
   }
   for (const auto &bk : b->buckets) {
     a.i0 = bk.i0;
     a.i1 = bk.i1;
-    cudaError_t e = launch_rnp_step_fp32(b->P, b->D, b->T, a, bk.decomp, b->stream);
+    cudaError_t e = launch_rnp_step_fp32(b->P, b->D, a, bk.decomp, b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "batched step launch");
   }
   return NLM_OK;
@@ -540,6 +540,12 @@ int nlm_batch_create(const nlm_fd_desc *descs, int nspec, nlm_batch **out) {
   D.bct = dbct;
   D.slice_spec = dss;
   D.flags = dflags;
+  if (any_nofail) {
+    uint8_t *marked;
+    BTRY(b->alloc(&marked, N));
+    BTRY(mark_rim(N, D.rowptr, D.cols, dflags, marked, st));
+    D.flags = marked;
+  }
   D.bcref = dbcref;
   D.bce = dbce;
   D.vol64 = vol64;
@@ -626,9 +632,9 @@ int nlm_batch_create(const nlm_fd_desc *descs, int nspec, nlm_batch **out) {
         if (b->tile_ok) cands.push_back(NLM_DECOMP_TILE_LOCAL);
         for (int c : cands) {
           StepArgs a{0, false, 0., b->dt, nullptr, bk.i0, bk.i1};
-          for (int w = 0; w < 2; w++) e2 = launch_rnp_step_fp32(P, Dt, b->T, a, c, st);
+          for (int w = 0; w < 2; w++) e2 = launch_rnp_step_fp32(P, Dt, a, c, st);
           cudaEventRecord(ea, st);
-          for (int r = 0; r < 3; r++) e2 = launch_rnp_step_fp32(P, Dt, b->T, a, c, st);
+          for (int r = 0; r < 3; r++) e2 = launch_rnp_step_fp32(P, Dt, a, c, st);
           cudaEventRecord(eb, st);
           if (e2 == cudaSuccess) e2 = cudaEventSynchronize(eb);
           float ms = 0.f;

@@ -64,7 +64,8 @@ enum : uint8_t {
   FLAG_FIX_Z = 4,
   FLAG_NOFAIL = 8,  // non-interior node: bonds never break (rnpBond.cpp:235-240)
   FLAG_FBC = 16,    // node carries an external force (Force_BC)
-  FLAG_GHOST = 32   // padding node of a batched specimen (never updated)
+  FLAG_GHOST = 32,  // padding node of a batched specimen (never updated)
+  FLAG_RIM = 64     // non-interior node, or a neighbour is (set by mark_rim)
 };
 
 constexpr int kMaxBCSets = 32;
@@ -75,6 +76,12 @@ constexpr int kMaxRow = 512;  // longest neighbour row the builder accepts
 struct BCTime {
   int fn;
   double p[4];
+};
+
+struct FBCItem {   // one Force_BC set acting on a node
+  int set;
+  int dir_mask;
+  double spatial;
 };
 
 struct BCEntry {   // one node with at least one prescribed dof

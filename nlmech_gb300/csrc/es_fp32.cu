@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128)
 template <int DIM, int SCHEME>
 __global__ void __launch_bounds__(128)
     k_es_force32(const StepParams P, const Params32 Q, const ESConst32 E, const DevPtrs D,
-                 const BCTable T, const StepArgs A) {
+                 const StepArgs A) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const float4 *ucur = D.u32[A.cur];
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128)
     fi[1] = fmaf(s, Y[1], fi[1]);
     if (DIM == 3) fi[2] = fmaf(s, Y[2], fi[2]);
   }
-  integrate_node32<DIM, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  integrate_node32<DIM, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // ---- tile-frame variants (NLM_DECOMP_TILE_LOCAL) ---------------------------
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kTileNodes)
 template <int DIM, int SCHEME>
 __global__ void __launch_bounds__(kTileNodes, 4)
     k_es_force32_tile(const StepParams P, const Params32 Q, const ESConst32 E, const DevPtrs D,
-                      const BCTable T, const StepArgs A) {
+                      const StepArgs A) {
   extern __shared__ float4 es_sm[];
   float4 *s_x = es_sm, *s_u = es_sm + D.tile_nmax;
   float *s_b = reinterpret_cast<float *>(es_sm + 2 * D.tile_nmax);
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kTileNodes, 4)
   fi[0] = __fadd_rn(fx.x, fx.y);
   fi[1] = __fadd_rn(fy.x, fy.y);
   if (DIM == 3) fi[2] = __fadd_rn(fz.x, fz.y);
-  integrate_node32<DIM, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  integrate_node32<DIM, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // Above 48 KB a kernel's dynamic shared memory must be opted into; each
@@ -524,8 +524,7 @@ static void es_tile_smem(K kernel, std::atomic<uint64_t> &done) {
 }
 
 template <int DIM>
-static cudaError_t es32_tile(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                             const StepArgs &a, cudaStream_t s) {
+static cudaError_t es32_tile(const StepParams &P, const DevPtrs &D, const StepArgs &a, cudaStream_t s) {
   const Params32 Q = make_p32(P);
   const ESConst32 E = make_es32(P);
   const unsigned g = (unsigned)((P.n + kTileNodes - 1) / kTileNodes);
@@ -536,25 +535,24 @@ static cudaError_t es32_tile(const StepParams &P, const DevPtrs &D, const BCTabl
   k_es_dil32_tile<DIM><<<g, kTileNodes, b1, s>>>(P, Q, E, D, a);
   if (P.scheme == NLM_VELOCITY_VERLET) {
     es_tile_smem(k_es_force32_tile<DIM, NLM_VELOCITY_VERLET>, opt_v);
-    k_es_force32_tile<DIM, NLM_VELOCITY_VERLET><<<g, kTileNodes, b2, s>>>(P, Q, E, D, T, a);
+    k_es_force32_tile<DIM, NLM_VELOCITY_VERLET><<<g, kTileNodes, b2, s>>>(P, Q, E, D, a);
   } else {
     es_tile_smem(k_es_force32_tile<DIM, NLM_CENTRAL_DIFFERENCE>, opt_c);
-    k_es_force32_tile<DIM, NLM_CENTRAL_DIFFERENCE><<<g, kTileNodes, b2, s>>>(P, Q, E, D, T, a);
+    k_es_force32_tile<DIM, NLM_CENTRAL_DIFFERENCE><<<g, kTileNodes, b2, s>>>(P, Q, E, D, a);
   }
   return cudaGetLastError();
 }
 
 template <int DIM>
-static cudaError_t es32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                        const StepArgs &a, cudaStream_t s) {
+static cudaError_t es32(const StepParams &P, const DevPtrs &D, const StepArgs &a, cudaStream_t s) {
   const Params32 Q = make_p32(P);
   const ESConst32 E = make_es32(P);
   const unsigned g = (unsigned)((P.n + 127) / 128);
   k_es_dil32<DIM><<<g, 128, 0, s>>>(P, Q, E, D, a);
   if (P.scheme == NLM_VELOCITY_VERLET)
-    k_es_force32<DIM, NLM_VELOCITY_VERLET><<<g, 128, 0, s>>>(P, Q, E, D, T, a);
+    k_es_force32<DIM, NLM_VELOCITY_VERLET><<<g, 128, 0, s>>>(P, Q, E, D, a);
   else
-    k_es_force32<DIM, NLM_CENTRAL_DIFFERENCE><<<g, 128, 0, s>>>(P, Q, E, D, T, a);
+    k_es_force32<DIM, NLM_CENTRAL_DIFFERENCE><<<g, 128, 0, s>>>(P, Q, E, D, a);
   return cudaGetLastError();
 }
 
@@ -571,12 +569,11 @@ cudaError_t launch_es_minv32(const double *mw, float *minv, int64_t n, cudaStrea
   return cudaGetLastError();
 }
 
-cudaError_t launch_es_step_fp32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                const StepArgs &a, int decomp, cudaStream_t s) {
+cudaError_t launch_es_step_fp32(const StepParams &P, const DevPtrs &D, const StepArgs &a, int decomp, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
   if (decomp == NLM_DECOMP_TILE_LOCAL && D.tile_lidx && D.tile_nmax > 0)
-    return P.dim == 2 ? es32_tile<2>(P, D, T, a, s) : es32_tile<3>(P, D, T, a, s);
-  return P.dim == 2 ? es32<2>(P, D, T, a, s) : es32<3>(P, D, T, a, s);
+    return P.dim == 2 ? es32_tile<2>(P, D, a, s) : es32_tile<3>(P, D, a, s);
+  return P.dim == 2 ? es32<2>(P, D, a, s) : es32<3>(P, D, a, s);
 }
 
 }  // namespace nlm

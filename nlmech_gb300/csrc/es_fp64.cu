@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(128)
 
 template <int DIM, int SCHEME>
 __global__ void __launch_bounds__(128)
-    k_es_force64(const StepParams P, const DevPtrs D, const BCTable T, const StepArgs A) {
+    k_es_force64(const StepParams P, const DevPtrs D, const StepArgs A) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const double *ucur = D.u64[A.cur];
@@ -114,9 +114,9 @@ __global__ void __launch_bounds__(128)
     if (DIM == 3) fi[2] = fi[2] + (Y[2] / Yl) * s;
   }
   if (A.first)
-    integrate_node64<DIM, SCHEME, true>(P, D, T, A, i, fl, ui, fi);
+    integrate_node64<DIM, SCHEME, true>(P, D, A, i, fl, ui, fi);
   else
-    integrate_node64<DIM, SCHEME, false>(P, D, T, A, i, fl, ui, fi);
+    integrate_node64<DIM, SCHEME, false>(P, D, A, i, fl, ui, fi);
 }
 
 // ---- the two passes over the FP64 bond store ----------------------------------
@@ -246,7 +246,7 @@ __device__ __forceinline__ double es_t64_coef(const double2 c, double theta, dou
 
 template <int DIM, int SCHEME, int G>
 __global__ void __launch_bounds__(128)
-    k_es_force64_bond(const StepParams P, const DevPtrs D, const BCTable T, const StepArgs A) {
+    k_es_force64_bond(const StepParams P, const DevPtrs D, const StepArgs A) {
   constexpr int U = G == 16 ? 1 : 2, W = G * U;
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   if (i >= P.n) return;
@@ -303,9 +303,9 @@ __global__ void __launch_bounds__(128)
   ld_node<DIM>(D.u64[A.cur], i, ui);
   const uint8_t fl = D.flags[i];
   if (A.first)
-    integrate_node64<DIM, SCHEME, true>(P, D, T, A, i, fl, ui, fi);
+    integrate_node64<DIM, SCHEME, true>(P, D, A, i, fl, ui, fi);
   else
-    integrate_node64<DIM, SCHEME, false>(P, D, T, A, i, fl, ui, fi);
+    integrate_node64<DIM, SCHEME, false>(P, D, A, i, fl, ui, fi);
 }
 
 cudaError_t launch_es_store64(const StepParams &P, const DevPtrs &D, cudaStream_t s) {
@@ -318,8 +318,7 @@ cudaError_t launch_es_store64(const StepParams &P, const DevPtrs &D, cudaStream_
 }
 
 template <int DIM>
-static cudaError_t es64(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                        const StepArgs &a, cudaStream_t s) {
+static cudaError_t es64(const StepParams &P, const DevPtrs &D, const StepArgs &a, cudaStream_t s) {
   const unsigned g = (unsigned)((P.n + 127) / 128);
   if (D.es64_x) {
     const int G = team64(P.n);
@@ -330,7 +329,7 @@ static cudaError_t es64(const StepParams &P, const DevPtrs &D, const BCTable &T,
       constexpr int N = decltype(team)::value;
       k_es_dil64_bond<DIM, N><<<gg, kTeamBlock, 0, s>>>(P, D);
       (vv ? k_es_force64_bond<DIM, NLM_VELOCITY_VERLET, N>
-          : k_es_force64_bond<DIM, NLM_CENTRAL_DIFFERENCE, N>)<<<gg, kTeamBlock, 0, s>>>(P, D, T, a);
+          : k_es_force64_bond<DIM, NLM_CENTRAL_DIFFERENCE, N>)<<<gg, kTeamBlock, 0, s>>>(P, D, a);
     };
     if (G == 1)
       run(std::integral_constant<int, 1>{});
@@ -344,17 +343,16 @@ static cudaError_t es64(const StepParams &P, const DevPtrs &D, const BCTable &T,
   }
   k_es_dil64<DIM><<<g, 128, 0, s>>>(P, D, a);
   if (P.scheme == NLM_VELOCITY_VERLET)
-    k_es_force64<DIM, NLM_VELOCITY_VERLET><<<g, 128, 0, s>>>(P, D, T, a);
+    k_es_force64<DIM, NLM_VELOCITY_VERLET><<<g, 128, 0, s>>>(P, D, a);
   else
-    k_es_force64<DIM, NLM_CENTRAL_DIFFERENCE><<<g, 128, 0, s>>>(P, D, T, a);
+    k_es_force64<DIM, NLM_CENTRAL_DIFFERENCE><<<g, 128, 0, s>>>(P, D, a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_es_step_fp64(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                const StepArgs &a, int decomp, cudaStream_t s) {
+cudaError_t launch_es_step_fp64(const StepParams &P, const DevPtrs &D, const StepArgs &a, int decomp, cudaStream_t s) {
   (void)decomp;
   if (P.n == 0) return cudaSuccess;
-  return P.dim == 2 ? es64<2>(P, D, T, a, s) : es64<3>(P, D, T, a, s);
+  return P.dim == 2 ? es64<2>(P, D, a, s) : es64<3>(P, D, a, s);
 }
 
 cudaError_t launch_es_setup(const StepParams &P, const DevPtrs &D, double *mw, cudaStream_t s) {

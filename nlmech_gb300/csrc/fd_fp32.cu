@@ -115,8 +115,7 @@ __device__ __forceinline__ float rnp_bond32(const Params32 &Q, const Node32<DIM>
 // together, so each thread keeps several independent loads in flight.
 template <int DIM, int SCHEME, bool NW1, int OPT, bool BATCH>
 __global__ void __launch_bounds__(128, DIM == 2 ? 7 : 5)
-    k_rnp32_thread(const StepParams P, const Params32 Q0, const DevPtrs D, const BCTable T,
-                   const StepArgs A) {
+    k_rnp32_thread(const StepParams P, const Params32 Q0, const DevPtrs D, const StepArgs A) {
   const int64_t i = A.i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= A.i1) return;
   if (BATCH && (D.flags[i] & FLAG_GHOST)) return;
@@ -170,14 +169,13 @@ __global__ void __launch_bounds__(128, DIM == 2 ? 7 : 5)
     }
   }
   if (nw) D.bits[NW1 ? i : (int64_t)((len - 1) >> 5) * P.npad + i] = word | nw;
-  integrate_node32<DIM, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  integrate_node32<DIM, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // Same decomposition without the four-wide grouping (one bond per iteration).
 template <int DIM, int SCHEME, bool NW1, int OPT, bool BATCH>
 __global__ void __launch_bounds__(128, DIM == 2 ? 12 : 8)
-    k_rnp32_thread1(const StepParams P, const Params32 Q0, const DevPtrs D, const BCTable T,
-                    const StepArgs A) {
+    k_rnp32_thread1(const StepParams P, const Params32 Q0, const DevPtrs D, const StepArgs A) {
   const int64_t i = A.i0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= A.i1) return;
   if (BATCH && (D.flags[i] & FLAG_GHOST)) return;
@@ -216,14 +214,13 @@ __global__ void __launch_bounds__(128, DIM == 2 ? 12 : 8)
     if (DIM == 3) fi[2] = fmaf(s, dv[2], fi[2]);
   }
   if (nw) D.bits[NW1 ? i : (int64_t)((len - 1) >> 5) * P.npad + i] = word | nw;
-  integrate_node32<DIM, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  integrate_node32<DIM, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // Warp-per-node over CSR rows; lane k of the warp owns bonds k, k+32, ...
 template <int DIM, int SCHEME, int OPT, bool BATCH>
 __global__ void __launch_bounds__(256)
-    k_rnp32_warp(const StepParams P, const Params32 Q0, const DevPtrs D, const BCTable T,
-                 const StepArgs A) {
+    k_rnp32_warp(const StepParams P, const Params32 Q0, const DevPtrs D, const StepArgs A) {
   const int64_t i = A.i0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= A.i1) return;
@@ -267,7 +264,7 @@ __global__ void __launch_bounds__(256)
     fi[1] += __shfl_xor_sync(0xffffffffu, fi[1], o);
     if (DIM == 3) fi[2] += __shfl_xor_sync(0xffffffffu, fi[2], o);
   }
-  if (lane == 0) integrate_node32<DIM, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  if (lane == 0) integrate_node32<DIM, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // Tile kernel (2-D): a block stages the positions and displacements of its
@@ -287,8 +284,7 @@ __device__ __forceinline__ void node_from_f4(const float4 a, Node32<2> &n) {
 
 template <int SCHEME, bool NW1, int OPT>
 __global__ void __launch_bounds__(kTileNodes, 3)
-    k_rnp32_tile(const StepParams P, const Params32 Q, const DevPtrs D, const BCTable T,
-                 const StepArgs A) {
+    k_rnp32_tile(const StepParams P, const Params32 Q, const DevPtrs D, const StepArgs A) {
   __shared__ float4 s_pos[kTileMaxLocal];
   __shared__ float4 s_u[kTileMaxLocal];
   __shared__ uint8_t s_fl[(OPT & OPT_NOFAIL) ? kTileMaxLocal : 1];
@@ -362,7 +358,7 @@ __global__ void __launch_bounds__(kTileNodes, 3)
     }
   }
   if (nw) D.bits[NW1 ? i : (int64_t)((len - 1) >> 5) * P.npad + i] = word | nw;
-  integrate_node32<2, SCHEME>(P, Q, D, T, A, i, fl, uih, uil, fi);
+  integrate_node32<2, SCHEME>(P, Q, D, A, i, fl, uih, uil, fi);
 }
 
 // Tile kernel with the bond data in the tile's own frame (2-D): staging
@@ -522,12 +518,16 @@ __device__ __forceinline__ void tile_bond_data(const TileShared &S, uint32_t o, 
 // bond-state bits; then the integrator epilogue.
 template <int SCHEME, bool NW1, int OPT, bool BATCH, bool UV, bool EXACT>
 __device__ __forceinline__ void tilel_node(const StepParams &P, const Params32 &Qn,
-                                           const DevPtrs &D, const BCTable &T, const StepArgs &A,
+                                           const DevPtrs &D, const StepArgs &A,
                                            const TileShared &S, const uint2 *sb, int64_t i, int il,
                                            uint8_t fl, int len, int nint, uint32_t word,
                                            float4 ui4, const float4 *vpre, const float2 *fpre) {
   constexpr bool KV = !(OPT & OPT_CONTACT) && !BATCH;
-  constexpr bool FAST = !(OPT & (OPT_NOFAIL | OPT_CONTACT));
+  // rows without broken bonds take the break-free loop, in a model with a
+  // no-fail region those whose bonds can all break (613 x 347 plate, horizon
+  // 4h, a rim of 8h and a force load: 19.4 us per step, 21.4 with every row in
+  // the full loop)
+  constexpr bool FAST = !(OPT & OPT_CONTACT);
   const int ng = (len + 3) >> 2;
   const float4 xi = reinterpret_cast<const float4 *>(S.xu)[il];
   const float2 xi_x = make_float2(xi.x, xi.y), xi_u = make_float2(xi.z, xi.w);
@@ -541,7 +541,7 @@ __device__ __forceinline__ void tilel_node(const StepParams &P, const Params32 &
   if (FAST) {
     if (!NW1)
       for (int w = 0; w * 32 < len; w++) word |= D.bits[(int64_t)w * P.npad + i];
-    full = word != 0u;
+    full = word != 0u || ((OPT & OPT_NOFAIL) && (fl & FLAG_RIM));
   }
   if (FAST && !full && !EXACT) {
     // bonds in pairs (lane x: bonds 0, 2 of a group; lane y: bonds 1, 3),
@@ -570,8 +570,15 @@ __device__ __forceinline__ void tilel_node(const StepParams &P, const Params32 &
         tile_bond_pair<OPT, KV, UV, IN>(Qn, dx, dy, ex, ey,
                                         make_float2(vj[2 * p], vj[2 * p + 1]), s1, bs2);
         mx = fmax3(mx, bs2.x, bs2.y);
-        fx = __ffma2_rn(s1, dx, fx);
-        fy = __ffma2_rn(s1, dy, fy);
+        if (OPT & OPT_NOFAIL) {
+          // bond by bond: the order of the full loop, which rows of such a
+          // model took before, so that their force is the same value
+          fi[0] = fmaf(s1.y, dx.y, fmaf(s1.x, dx.x, fi[0]));
+          fi[1] = fmaf(s1.y, dy.y, fmaf(s1.x, dy.x, fi[1]));
+        } else {
+          fx = __ffma2_rn(s1, dx, fx);
+          fy = __ffma2_rn(s1, dy, fy);
+        }
       }
     };
     const int gi = min(nint >> 2, ng);
@@ -588,8 +595,10 @@ __device__ __forceinline__ void tilel_node(const StepParams &P, const Params32 &
       if (g + 1 < ng) nxt = sb[32 * (g + 1)];
       group(cur, std::false_type{});
     }
-    fi[0] = __fadd_rn(fx.x, fx.y);
-    fi[1] = __fadd_rn(fy.x, fy.y);
+    if (!(OPT & OPT_NOFAIL)) {
+      fi[0] = __fadd_rn(fx.x, fx.y);
+      fi[1] = __fadd_rn(fy.x, fy.y);
+    }
     full = mx > Qn.ksc_on;
   } else if (FAST && !full) {
     float mx = 0.f;  // largest S^2 r of the row
@@ -670,13 +679,12 @@ __device__ __forceinline__ void tilel_node(const StepParams &P, const Params32 &
     if (len & 31) nw &= (1u << (len & 31)) - 1u;
     if (nw) D.bits[NW1 ? i : (int64_t)((len - 1) >> 5) * P.npad + i] = word | nw;
   }
-  integrate_node32<2, SCHEME>(P, Qn, D, T, A, i, fl, uih, uil, fi, vpre, fpre);
+  integrate_node32<2, SCHEME, !BATCH>(P, Qn, D, A, i, fl, uih, uil, fi, vpre, fpre);
 }
 
 template <int SCHEME, bool NW1, int OPT, bool BATCH, bool UV>
 __global__ void __launch_bounds__(kTileNodes, 4)
-    k_rnp32_tilel(const StepParams P, const Params32 Q, const DevPtrs D, const BCTable T,
-                  const StepArgs A) {
+    k_rnp32_tilel(const StepParams P, const Params32 Q, const DevPtrs D, const StepArgs A) {
   // per staged node: x - x_o, y - y_o, and ux - ux_o, uy - uy_o (frame mode)
   // or the hi parts of ux, uy (exact mode, lo parts in s_ul)
   __shared__ float4 s_xu[kTileMaxLocal];
@@ -835,10 +843,10 @@ __global__ void __launch_bounds__(kTileNodes, 4)
   const TileShared S{reinterpret_cast<const char *>(s_xu), reinterpret_cast<const char *>(s_vol),
                      reinterpret_cast<const char *>(s_ul), s_fl};
   if (exact)
-    tilel_node<SCHEME, NW1, OPT, BATCH, UV, true>(P, Qn, D, T, A, S, sb, i, il, fl, len, nint,
+    tilel_node<SCHEME, NW1, OPT, BATCH, UV, true>(P, Qn, D, A, S, sb, i, il, fl, len, nint,
                                                   word, ui4, vp, fp);
   else
-    tilel_node<SCHEME, NW1, OPT, BATCH, UV, false>(P, Qn, D, T, A, S, sb, i, il, fl, len, nint,
+    tilel_node<SCHEME, NW1, OPT, BATCH, UV, false>(P, Qn, D, A, S, sb, i, il, fl, len, nint,
                                                    word, ui4, vp, fp);
 }
 
@@ -860,29 +868,29 @@ static void tile_ids_smem(K kernel, std::atomic<uint64_t> &done) {
 // reads after the previous step).
 template <class K>
 static void tilel_go(K kernel, const StepParams &P, const Params32 &Q, const DevPtrs &D,
-                     const BCTable &T, const StepArgs &a, unsigned grid, size_t dyn,
+                     const StepArgs &a, unsigned grid, size_t dyn,
                      cudaStream_t s) {
-  launch_pdl(kernel, grid, kTileNodes, dyn, s, a.pdl, P, Q, D, T, a);
+  launch_pdl(kernel, grid, kTileNodes, dyn, s, a.pdl, P, Q, D, a);
 }
 
 template <int SCHEME, int OPT, bool BATCH, bool UV>
 static void tilel_launch(const StepParams &P, const Params32 &Q, const DevPtrs &D,
-                         const BCTable &T, const StepArgs &a, unsigned grid, size_t dyn,
+                         const StepArgs &a, unsigned grid, size_t dyn,
                          cudaStream_t s) {
   if (P.nw1) {
     static std::atomic<uint64_t> opt{0};
     tile_ids_smem(k_rnp32_tilel<SCHEME, true, OPT, BATCH, UV>, opt);
-    tilel_go(k_rnp32_tilel<SCHEME, true, OPT, BATCH, UV>, P, Q, D, T, a, grid, dyn, s);
+    tilel_go(k_rnp32_tilel<SCHEME, true, OPT, BATCH, UV>, P, Q, D, a, grid, dyn, s);
   } else {
     static std::atomic<uint64_t> opt{0};
     tile_ids_smem(k_rnp32_tilel<SCHEME, false, OPT, BATCH, UV>, opt);
-    tilel_go(k_rnp32_tilel<SCHEME, false, OPT, BATCH, UV>, P, Q, D, T, a, grid, dyn, s);
+    tilel_go(k_rnp32_tilel<SCHEME, false, OPT, BATCH, UV>, P, Q, D, a, grid, dyn, s);
   }
 }
 
 template <int DIM, int SCHEME, int OPT, bool BATCH>
 static void launch_opt(const StepParams &P, const Params32 &Q, const DevPtrs &D,
-                       const BCTable &T, const StepArgs &a, int decomp, cudaStream_t s) {
+                       const StepArgs &a, int decomp, cudaStream_t s) {
   const int64_t nodes = a.i1 - a.i0;
   if (nodes <= 0) return;
   if (DIM == 2 && !BATCH && decomp == NLM_DECOMP_TILE) {
@@ -892,9 +900,9 @@ static void launch_opt(const StepParams &P, const Params32 &Q, const DevPtrs &D,
         a.tiles ? (unsigned)a.ntiles : (unsigned)((P.n + kTileNodes - 1) / kTileNodes);
     if (grid == 0) return;
     if (P.nw1)
-      k_rnp32_tile<SCHEME, true, OPT><<<grid, kTileNodes, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_tile<SCHEME, true, OPT><<<grid, kTileNodes, 0, s>>>(P, Q, D, a);
     else
-      k_rnp32_tile<SCHEME, false, OPT><<<grid, kTileNodes, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_tile<SCHEME, false, OPT><<<grid, kTileNodes, 0, s>>>(P, Q, D, a);
     return;
   }
   if (DIM == 2 && decomp == NLM_DECOMP_TILE_LOCAL && D.tile_boff) {
@@ -909,36 +917,35 @@ static void launch_opt(const StepParams &P, const Params32 &Q, const DevPtrs &D,
     // constants in each specimen's table): K1 V as a constant
     constexpr bool UVOK = !(OPT & OPT_CONTACT);
     if (UVOK && (BATCH ? P.uv_specimens != 0 : Q.kv_uniform > 0.f)) {
-      tilel_launch<SCHEME, OPT, BATCH, UVOK>(P, Q, D, T, a, grid, dyn, s);
+      tilel_launch<SCHEME, OPT, BATCH, UVOK>(P, Q, D, a, grid, dyn, s);
     } else {
-      tilel_launch<SCHEME, OPT, BATCH, false>(P, Q, D, T, a, grid, dyn, s);
+      tilel_launch<SCHEME, OPT, BATCH, false>(P, Q, D, a, grid, dyn, s);
     }
     return;
   }
   if (decomp == NLM_DECOMP_WARP) {
     const int bs = 256;
     const unsigned grid = (unsigned)((nodes * 32 + bs - 1) / bs);
-    k_rnp32_warp<DIM, SCHEME, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, T, a);
+    k_rnp32_warp<DIM, SCHEME, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, a);
     return;
   }
   const int bs = 128;
   const unsigned grid = (unsigned)((nodes + bs - 1) / bs);
   if (decomp == NLM_DECOMP_THREAD1) {
     if (P.nw1)
-      k_rnp32_thread1<DIM, SCHEME, true, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_thread1<DIM, SCHEME, true, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, a);
     else
-      k_rnp32_thread1<DIM, SCHEME, false, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_thread1<DIM, SCHEME, false, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, a);
   } else {
     if (P.nw1)
-      k_rnp32_thread<DIM, SCHEME, true, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_thread<DIM, SCHEME, true, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, a);
     else
-      k_rnp32_thread<DIM, SCHEME, false, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, T, a);
+      k_rnp32_thread<DIM, SCHEME, false, OPT, BATCH><<<grid, bs, 0, s>>>(P, Q, D, a);
   }
 }
 
 template <int DIM, int SCHEME>
-static cudaError_t launch32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                            const StepArgs &a, int decomp, cudaStream_t s) {
+static cudaError_t launch32(const StepParams &P, const DevPtrs &D, const StepArgs &a, int decomp, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
   const Params32 Q = make_p32(P);
   const int opt = (P.infl_type == 0 ? OPT_CONSTJ : 0) | (P.nofail ? OPT_NOFAIL : 0) |
@@ -948,38 +955,37 @@ static cudaError_t launch32(const StepParams &P, const DevPtrs &D, const BCTable
     // specimens may mix influence functions: the batch path always takes the
     // general influence evaluation
     if (P.nofail)
-      launch_opt<DIM, SCHEME, OPT_NOFAIL, true>(P, Q, D, T, a, decomp, s);
+      launch_opt<DIM, SCHEME, OPT_NOFAIL, true>(P, Q, D, a, decomp, s);
     else
-      launch_opt<DIM, SCHEME, 0, true>(P, Q, D, T, a, decomp, s);
+      launch_opt<DIM, SCHEME, 0, true>(P, Q, D, a, decomp, s);
     return cudaGetLastError();
   }
   switch (opt) {
-    case 0: launch_opt<DIM, SCHEME, 0, false>(P, Q, D, T, a, decomp, s); break;
-    case 1: launch_opt<DIM, SCHEME, 1, false>(P, Q, D, T, a, decomp, s); break;
-    case 2: launch_opt<DIM, SCHEME, 2, false>(P, Q, D, T, a, decomp, s); break;
-    case 3: launch_opt<DIM, SCHEME, 3, false>(P, Q, D, T, a, decomp, s); break;
-    case 4: launch_opt<DIM, SCHEME, 4, false>(P, Q, D, T, a, decomp, s); break;
-    case 5: launch_opt<DIM, SCHEME, 5, false>(P, Q, D, T, a, decomp, s); break;
-    case 6: launch_opt<DIM, SCHEME, 6, false>(P, Q, D, T, a, decomp, s); break;
-    default: launch_opt<DIM, SCHEME, 7, false>(P, Q, D, T, a, decomp, s); break;
+    case 0: launch_opt<DIM, SCHEME, 0, false>(P, Q, D, a, decomp, s); break;
+    case 1: launch_opt<DIM, SCHEME, 1, false>(P, Q, D, a, decomp, s); break;
+    case 2: launch_opt<DIM, SCHEME, 2, false>(P, Q, D, a, decomp, s); break;
+    case 3: launch_opt<DIM, SCHEME, 3, false>(P, Q, D, a, decomp, s); break;
+    case 4: launch_opt<DIM, SCHEME, 4, false>(P, Q, D, a, decomp, s); break;
+    case 5: launch_opt<DIM, SCHEME, 5, false>(P, Q, D, a, decomp, s); break;
+    case 6: launch_opt<DIM, SCHEME, 6, false>(P, Q, D, a, decomp, s); break;
+    default: launch_opt<DIM, SCHEME, 7, false>(P, Q, D, a, decomp, s); break;
   }
   return cudaGetLastError();
 }
 
-cudaError_t launch_rnp_step_fp32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                 const StepArgs &a, int decomp, cudaStream_t s) {
+cudaError_t launch_rnp_step_fp32(const StepParams &P, const DevPtrs &D, const StepArgs &a, int decomp, cudaStream_t s) {
   if (P.dim == 2)
-    return P.scheme == NLM_VELOCITY_VERLET ? launch32<2, NLM_VELOCITY_VERLET>(P, D, T, a, decomp, s)
-                                           : launch32<2, NLM_CENTRAL_DIFFERENCE>(P, D, T, a, decomp, s);
-  return P.scheme == NLM_VELOCITY_VERLET ? launch32<3, NLM_VELOCITY_VERLET>(P, D, T, a, decomp, s)
-                                         : launch32<3, NLM_CENTRAL_DIFFERENCE>(P, D, T, a, decomp, s);
+    return P.scheme == NLM_VELOCITY_VERLET ? launch32<2, NLM_VELOCITY_VERLET>(P, D, a, decomp, s)
+                                           : launch32<2, NLM_CENTRAL_DIFFERENCE>(P, D, a, decomp, s);
+  return P.scheme == NLM_VELOCITY_VERLET ? launch32<3, NLM_VELOCITY_VERLET>(P, D, a, decomp, s)
+                                         : launch32<3, NLM_CENTRAL_DIFFERENCE>(P, D, a, decomp, s);
 }
 
 // One node's drift from the state (u, v, f) of the last step: the second
 // half of integrate_node32, prescribed dofs from the loading at t_next.
 template <int DIM>
 __device__ __forceinline__ void drift_node32(const StepParams &P, const Params32 &Q,
-                                             const DevPtrs &D, const BCTable &T, uint8_t fl,
+                                             const DevPtrs &D, uint8_t fl,
                                              int ref, const float uh[3], const float ul[3],
                                              const float vh[3], const float vl[3],
                                              const float f[3], double t_next, df un[3],
@@ -996,7 +1002,7 @@ __device__ __forceinline__ void drift_node32(const StepParams &P, const Params32
         vn[c] = df_mul_c(df_sub(un[c], u), Q.idt_hi, Q.idt_lo);
       }
     } else {
-      bc_df(D, T, ref, c, t_next, un[c], vn[c]);
+      bc_df(D, ref, c, t_next, un[c], vn[c]);
     }
   }
 }
@@ -1004,7 +1010,7 @@ __device__ __forceinline__ void drift_node32(const StepParams &P, const Params32
 // Drift after a host state upload.
 template <int DIM>
 __global__ void k_drift32(const StepParams P, const Params32 Q, const DevPtrs D,
-                          const BCTable T, int cur, double t_next) {
+                          int cur, double t_next) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const uint8_t fl = D.flags[i];
@@ -1014,7 +1020,7 @@ __global__ void k_drift32(const StepParams P, const Params32 Q, const DevPtrs D,
   ld_pair<DIM>(D.v32[P.scheme == NLM_CENTRAL_DIFFERENCE ? cur : 0], i, vh, vl);
   for (int c = 0; c < DIM; c++) f[c] = D.f32[(int64_t)(DIM == 2 ? 2 : 4) * i + c];
   df un[3], vn[3];
-  drift_node32<DIM>(P, Q, D, T, fl, ref, uh, ul, vh, vl, f, t_next, un, vn);
+  drift_node32<DIM>(P, Q, D, fl, ref, uh, ul, vh, vl, f, t_next, un, vn);
   st_pair<DIM>(D.u32[1 - cur], i, un);
   if (P.scheme == NLM_CENTRAL_DIFFERENCE) st_pair<DIM>(D.v32[1 - cur], i, vn);
 }
@@ -1025,7 +1031,7 @@ __global__ void k_drift32(const StepParams P, const Params32 Q, const DevPtrs D,
 // kernel reads them -- with the same (hi, lo) splits as a whole-state upload,
 // and a flag for any non-finite value.
 __global__ void k_pipe_in32(const StepParams P, const Params32 Q, const DevPtrs D,
-                            const BCTable T, double t_next, int64_t o0, int64_t o1,
+                            double t_next, int64_t o0, int64_t o1,
                             const int *iperm, const double *hu, const double *hv,
                             const double *hf, float4 *ua, float4 *sv, float2 *sf, int *bad) {
   const int64_t o = o0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1053,7 +1059,7 @@ __global__ void k_pipe_in32(const StepParams P, const Params32 Q, const DevPtrs 
     fs[c] = __double2float_rn(f[c]);
   }
   df un[3], vn[3];
-  drift_node32<2>(P, Q, D, T, fl, ref, uh, ul, vh, vl, fs, t_next, un, vn);
+  drift_node32<2>(P, Q, D, fl, ref, uh, ul, vh, vl, fs, t_next, un, vn);
   st_pair<2>(ua, i, un);
   sv[i] = make_float4(vh[0], vh[1], vl[0], vl[1]);
   sf[i] = make_float2(fs[0], fs[1]);
@@ -1104,13 +1110,12 @@ __global__ void k_pipe_commit32(int64_t n, int64_t nbits, const int *bad, const 
   }
 }
 
-cudaError_t launch_pipe_in32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                             double t_next, int64_t o0, int64_t o1, const int *iperm,
+cudaError_t launch_pipe_in32(const StepParams &P, const DevPtrs &D, double t_next, int64_t o0, int64_t o1, const int *iperm,
                              const double *hu, const double *hv, const double *hf, float4 *ua,
                              float4 *sv, float2 *sf, int *bad, cudaStream_t s) {
   if (o1 <= o0) return cudaSuccess;
   const Params32 Q = make_p32(P);
-  k_pipe_in32<<<(unsigned)((o1 - o0 + 255) / 256), 256, 0, s>>>(P, Q, D, T, t_next, o0, o1,
+  k_pipe_in32<<<(unsigned)((o1 - o0 + 255) / 256), 256, 0, s>>>(P, Q, D, t_next, o0, o1,
                                                                  iperm, hu, hv, hf, ua, sv, sf,
                                                                  bad);
   return cudaGetLastError();
@@ -1138,15 +1143,15 @@ cudaError_t launch_pipe_commit32(int64_t n, int64_t nbits, const int *bad, const
   return cudaGetLastError();
 }
 
-cudaError_t launch_drift32(const StepParams &P, const DevPtrs &D, const BCTable &T, int cur,
+cudaError_t launch_drift32(const StepParams &P, const DevPtrs &D, int cur,
                            double t_next, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
   const Params32 Q = make_p32(P);
   const unsigned g = (unsigned)((P.n + 255) / 256);
   if (P.dim == 2)
-    k_drift32<2><<<g, 256, 0, s>>>(P, Q, D, T, cur, t_next);
+    k_drift32<2><<<g, 256, 0, s>>>(P, Q, D, cur, t_next);
   else
-    k_drift32<3><<<g, 256, 0, s>>>(P, Q, D, T, cur, t_next);
+    k_drift32<3><<<g, 256, 0, s>>>(P, Q, D, cur, t_next);
   return cudaGetLastError();
 }
 

@@ -78,7 +78,7 @@ __device__ __forceinline__ double contact64(const StepParams &P, const double xi
 // recomputed from the positions.
 template <int DIM, int SCHEME, bool FIRST>
 __global__ void __launch_bounds__(128)
-    k_rnp64_thread(const StepParams P, const DevPtrs D, const BCTable T, const StepArgs A) {
+    k_rnp64_thread(const StepParams P, const DevPtrs D, const StepArgs A) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const double *ucur = D.u64[A.cur];
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (dirty) D.bits[(int64_t)chunk * P.npad + i] = word;
-  integrate_node64<DIM, SCHEME, FIRST>(P, D, T, A, i, fl, ui, fi);
+  integrate_node64<DIM, SCHEME, FIRST>(P, D, A, i, fl, ui, fi);
 }
 
 // ---- step over the FP64 bond store ------------------------------------------
@@ -188,8 +188,7 @@ __global__ void k_rnp64_store(const StepParams P, const DevPtrs D, double2 *bd, 
 // here, 33 FP64 instructions per bond, the FP64 pipe 85 % busy: the bound.
 template <int DIM, int SCHEME, bool FIRST, int G>
 __global__ void __launch_bounds__(128)
-    k_rnp64_bond(const StepParams P, const double inv_invF, const DevPtrs D, const BCTable T,
-                 const StepArgs A) {
+    k_rnp64_bond(const StepParams P, const double inv_invF, const DevPtrs D, const StepArgs A) {
   constexpr int U = G == 16 ? 1 : 2, W = G * U;
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   if (i >= P.n) return;
@@ -289,7 +288,7 @@ __global__ void __launch_bounds__(128)
       if (c == 0) D.bits[(int64_t)(kb >> 5) * P.npad + i] = word;
     }
   }
-  if (c == 0) integrate_node64<DIM, SCHEME, FIRST>(P, D, T, A, i, D.flags[i], ui, fi);
+  if (c == 0) integrate_node64<DIM, SCHEME, FIRST>(P, D, A, i, D.flags[i], ui, fi);
 }
 
 // Teams pay the row-order additions G times but fill the chip where one thread
@@ -311,8 +310,7 @@ cudaError_t launch_rnp_store64(const StepParams &P, const DevPtrs &D, cudaStream
 }
 
 template <int DIM, int SCHEME>
-static cudaError_t launch_dim(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                              const StepArgs &a, cudaStream_t s) {
+static cudaError_t launch_dim(const StepParams &P, const DevPtrs &D, const StepArgs &a, cudaStream_t s) {
   const int bs = 128;
   const unsigned grid = (unsigned)((P.n + bs - 1) / bs);
   if (P.n == 0) return cudaSuccess;
@@ -328,22 +326,21 @@ static cudaError_t launch_dim(const StepParams &P, const DevPtrs &D, const BCTab
                       : k_rnp64_bond<DIM, SCHEME, F, 16>;
     };
     auto kern = a.first ? pick(std::true_type{}) : pick(std::false_type{});
-    kern<<<gg, kTeamBlock, 0, s>>>(P, inv, D, T, a);
+    kern<<<gg, kTeamBlock, 0, s>>>(P, inv, D, a);
   } else if (a.first)
-    k_rnp64_thread<DIM, SCHEME, true><<<grid, bs, 0, s>>>(P, D, T, a);
+    k_rnp64_thread<DIM, SCHEME, true><<<grid, bs, 0, s>>>(P, D, a);
   else
-    k_rnp64_thread<DIM, SCHEME, false><<<grid, bs, 0, s>>>(P, D, T, a);
+    k_rnp64_thread<DIM, SCHEME, false><<<grid, bs, 0, s>>>(P, D, a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_rnp_step_fp64(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                 const StepArgs &a, int decomp, cudaStream_t s) {
+cudaError_t launch_rnp_step_fp64(const StepParams &P, const DevPtrs &D, const StepArgs &a, int decomp, cudaStream_t s) {
   (void)decomp;  // every FP64 path keeps the reference summation order
   if (P.dim == 2)
-    return P.scheme == NLM_VELOCITY_VERLET ? launch_dim<2, NLM_VELOCITY_VERLET>(P, D, T, a, s)
-                                           : launch_dim<2, NLM_CENTRAL_DIFFERENCE>(P, D, T, a, s);
-  return P.scheme == NLM_VELOCITY_VERLET ? launch_dim<3, NLM_VELOCITY_VERLET>(P, D, T, a, s)
-                                         : launch_dim<3, NLM_CENTRAL_DIFFERENCE>(P, D, T, a, s);
+    return P.scheme == NLM_VELOCITY_VERLET ? launch_dim<2, NLM_VELOCITY_VERLET>(P, D, a, s)
+                                           : launch_dim<2, NLM_CENTRAL_DIFFERENCE>(P, D, a, s);
+  return P.scheme == NLM_VELOCITY_VERLET ? launch_dim<3, NLM_VELOCITY_VERLET>(P, D, a, s)
+                                         : launch_dim<3, NLM_CENTRAL_DIFFERENCE>(P, D, a, s);
 }
 
 // FDModel::computePostProcFields, damage part (fDModel.cpp:651-778):
@@ -597,7 +594,7 @@ namespace nlm {
 
 // Second half of integrate_node64 / integrate_node32 on its own.
 template <int DIM>
-__global__ void k_drift64(const StepParams P, const DevPtrs D, const BCTable T, int cur,
+__global__ void k_drift64(const StepParams P, const DevPtrs D, int cur,
                           double t_next) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= P.n) return;
@@ -620,7 +617,7 @@ __global__ void k_drift64(const StepParams P, const DevPtrs D, const BCTable T, 
       }
     } else {
       double du, dv;
-      bc_dof(D, T, ref, d, t_next, du, dv);
+      bc_dof(D, ref, d, t_next, du, dv);
       un[d] = du;
       vn[d] = dv;
     }
@@ -629,15 +626,15 @@ __global__ void k_drift64(const StepParams P, const DevPtrs D, const BCTable T, 
   if (P.scheme == NLM_CENTRAL_DIFFERENCE) st_node<DIM>(D.v[1 - cur], i, vn);
 }
 
-cudaError_t launch_drift(const StepParams &P, const DevPtrs &D, const BCTable &T, int cur,
+cudaError_t launch_drift(const StepParams &P, const DevPtrs &D, int cur,
                          double t_next, bool fp32, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  if (fp32) return launch_drift32(P, D, T, cur, t_next, s);
+  if (fp32) return launch_drift32(P, D, cur, t_next, s);
   const unsigned g = (unsigned)((P.n + 255) / 256);
   if (P.dim == 2)
-    k_drift64<2><<<g, 256, 0, s>>>(P, D, T, cur, t_next);
+    k_drift64<2><<<g, 256, 0, s>>>(P, D, cur, t_next);
   else
-    k_drift64<3><<<g, 256, 0, s>>>(P, D, T, cur, t_next);
+    k_drift64<3><<<g, 256, 0, s>>>(P, D, cur, t_next);
   return cudaGetLastError();
 }
 

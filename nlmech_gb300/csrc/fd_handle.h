@@ -49,13 +49,6 @@ double uload_umax(const nlm_bc_set &bc, const double *x);
 double fload_spatial(const nlm_bc_set &bc, const double *x, double h);
 
 // ---- small kernels (fd_kernels.cu) ---------------------------------------
-struct FBCItem {
-  int set;
-  int dir_mask;
-  double spatial;
-};
-
-
 __device__ inline void ld_split_any(const float4 *p, int S, int64_t i, double o[3]) {
   if (S == 2) {
     const float4 a = p[i];
@@ -84,8 +77,7 @@ __device__ inline void st_split_any(float4 *p, int S, int64_t i, const double v[
 }
 
 __global__ void k_fbc_apply(int64_t nf, int S, const int *nodes, const int *iptr,
-                            const FBCItem *items, BCTable T, double time, double *fext,
-                            const double *tdev = nullptr);
+                            const FBCItem *items, BCTable T, double time, double *fext);
 __global__ void k_bc_apply(int64_t nb, int S, int dim, const int *nodes, const int *bcref,
                            const BCEntry *bce, const uint8_t *flags, BCTable T, double time,
                            double *u64, float4 *u32, double *v, float4 *v32);

@@ -324,11 +324,11 @@ int launch_step(nlm_fd *h, const StepArgs &a0) {
   cudaError_t e;
   const bool fp32 = h->precision == NLM_PREC_FP32C;
   if (h->material == NLM_MAT_RNP_BOND)
-    e = fp32 ? launch_rnp_step_fp32(h->P, h->D, h->T, a, h->decomp, h->stream)
-             : launch_rnp_step_fp64(h->P, h->D, h->T, a, h->decomp, h->stream);
+    e = fp32 ? launch_rnp_step_fp32(h->P, h->D, a, h->decomp, h->stream)
+             : launch_rnp_step_fp64(h->P, h->D, a, h->decomp, h->stream);
   else
-    e = fp32 ? launch_es_step_fp32(h->P, h->D, h->T, a, h->decomp, h->stream)
-             : launch_es_step_fp64(h->P, h->D, h->T, a, h->decomp, h->stream);
+    e = fp32 ? launch_es_step_fp32(h->P, h->D, a, h->decomp, h->stream)
+             : launch_es_step_fp64(h->P, h->D, a, h->decomp, h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
   if (h->timing && !h->capturing) {
     NLM_CUDA(cudaEventRecord(e1, h->stream));
@@ -452,14 +452,16 @@ int autotune(nlm_fd *h) {
   float best = 1e30f;
   int pick = NLM_DECOMP_THREAD;
   StepArgs sa{0, false, h->time, h->time + h->dt, nullptr, 0, h->n};
+  sa.pdl = true;  // as the steps of a run are launched
+  const int reps = n < 100000 ? 25 : 5;  // 5 launches of 7 us differ by more than the candidates
   for (int c : cands) {
     auto launch = [&]() {
-      return rnp ? launch_rnp_step_fp32(h->P, D, h->T, sa, c, s)
-                 : launch_es_step_fp32(h->P, D, h->T, sa, c, s);
+      return rnp ? launch_rnp_step_fp32(h->P, D, sa, c, s)
+                 : launch_es_step_fp32(h->P, D, sa, c, s);
     };
     for (int w = 0; w < 2; w++) e = launch();
     cudaEventRecord(a, s);
-    for (int r = 0; r < 5; r++) e = launch();
+    for (int r = 0; r < reps; r++) e = launch();
     cudaEventRecord(b, s);
     if (e == cudaSuccess) e = cudaEventSynchronize(b);
     float ms = 0.f;
@@ -511,16 +513,8 @@ int capture_graph(nlm_fd *h, int c0) {
   int c = c0, rc = NLM_OK;
   for (int k = 0; k < h->graph_steps && rc == NLM_OK; k++) {
     c = 1 - c;
-    if (h->n_fbc_nodes > 0) {
-      // FLoading::apply at the step's time, read from the time array
-      k_fbc_apply<<<nblk(h->n_fbc_nodes, 128), 128, 0, h->stream>>>(
-          h->n_fbc_nodes, h->S, h->fbc_nodes, h->fbc_iptr, h->fbc_items, h->FT, 0.,
-          const_cast<double *>(h->D.fext), h->d_times + k);
-      const cudaError_t ef = cudaGetLastError();
-      if (ef != cudaSuccess) rc = cuda_fail(ef, "force-load kernel");
-    }
     StepArgs a{c, false, 0., 0., h->d_times + k, 0, h->n};
-    if (rc == NLM_OK) rc = launch_step(h, a);
+    rc = launch_step(h, a);
   }
   e = cudaStreamEndCapture(h->stream, &g);
   h->capturing = false;
@@ -571,7 +565,6 @@ int single_steps(nlm_fd *h, int64_t nsteps) {
     if (!h->timed_cracks.empty() && h->step > 0 && (rc = add_crack(h))) return rc;
     const double tm = h->time + h->dt;
     h->cur = 1 - h->cur;
-    if ((rc = apply_fbc(h, tm))) return rc;
     StepArgs a{h->cur, false, tm, tm + h->dt, nullptr, 0, h->n};
     if ((rc = launch_step(h, a))) return rc;
     h->time = tm;
@@ -584,7 +577,6 @@ int do_run(nlm_fd *h, int64_t nsteps) {
   if (!h->started) {
     int rc = apply_bc(h, h->time);
     if (rc) return rc;
-    if ((rc = apply_fbc(h, h->time))) return rc;
     StepArgs a{h->cur, true, h->time, h->time + h->dt, nullptr, 0, h->n};
     if ((rc = launch_step(h, a))) return rc;
     h->started = true;
@@ -974,8 +966,18 @@ int create_model(const nlm_fd_desc *d, nlm_fd **out, bool explicit_steps) {
   if (!bce.empty())
     TRY(cudaMemcpyAsync(dbce, bce.data(), sizeof(BCEntry) * bce.size(), cudaMemcpyHostToDevice, s));
   D.flags = dflags;
+  if (any_nofail && h->precision == NLM_PREC_FP32C) {
+    uint8_t *marked;
+    TRY(h->alloc(&marked, n));
+    TRY(mark_rim(n, D.rowptr, D.cols, dflags, marked, s));
+    D.flags = marked;
+  }
   D.bcref = dbcref;
   D.bce = dbce;
+  BCTime *dbct;
+  TRY(h->alloc(&dbct, kMaxBCSets));
+  TRY(cudaMemcpyAsync(dbct, h->T.t, sizeof(BCTime) * kMaxBCSets, cudaMemcpyHostToDevice, s));
+  D.bct = dbct;
   h->n_bc_nodes = (int64_t)bcn.size();
   TRY(h->alloc(&h->bc_nodes, bcn.size() + 1));
   if (!bcn.empty())
@@ -992,6 +994,19 @@ int create_model(const nlm_fd_desc *d, nlm_fd **out, bool explicit_steps) {
     TRY(cudaMemcpyAsync(h->fbc_nodes, fnodes.data(), sizeof(int) * fnodes.size(), cudaMemcpyHostToDevice, s));
     TRY(cudaMemcpyAsync(h->fbc_iptr, fptr.data(), sizeof(int) * fptr.size(), cudaMemcpyHostToDevice, s));
     TRY(cudaMemcpyAsync(h->fbc_items, fits.data(), sizeof(FBCItem) * fits.size(), cudaMemcpyHostToDevice, s));
+    std::vector<int> fref(n, -1);
+    for (size_t k = 0; k < fnodes.size(); k++) fref[fnodes[k]] = (int)k;
+    int *dref;
+    BCTime *dt;
+    TRY(h->alloc(&dref, n));
+    TRY(h->alloc(&dt, kMaxBCSets));
+    TRY(cudaMemcpyAsync(dref, fref.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    TRY(cudaMemcpyAsync(dt, h->FT.t, sizeof(BCTime) * kMaxBCSets, cudaMemcpyHostToDevice, s));
+    TRY(cudaStreamSynchronize(s));
+    D.fbc_ref = dref;
+    D.fbc_iptr = h->fbc_iptr;
+    D.fbc_items = h->fbc_items;
+    D.fbc_t = dt;
   }
   double *vol64;
   TRY(h->alloc(&vol64, n));

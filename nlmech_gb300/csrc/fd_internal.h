@@ -19,7 +19,12 @@ struct DevPtrs {
   const uint8_t *flags;
   const int *bcref;     // node -> BCEntry index (-1 none)
   const BCEntry *bce;
-  const double *fext;   // S doubles per node, valid where FLAG_FBC is set
+  const double *fext;   // S doubles per node, valid where FLAG_FBC is set (the
+                        // quasi-static models; a time step evaluates the loads)
+  const int *fbc_ref;   // node -> its entry of fbc_iptr (-1: none)
+  const int *fbc_iptr;  // items of an entry: fbc_iptr[e] .. fbc_iptr[e + 1]
+  const FBCItem *fbc_items;
+  const BCTime *fbc_t;  // time functions by set
   // topology
   const int64_t *sell_ptr;  // per 32-node slice: first entry
   const int *sell_w;        // per slice: width (longest row)
@@ -58,8 +63,10 @@ struct DevPtrs {
   float2 *es_ab;          // FP32C: t = a |X| + b e coefficients per node
   int *err;               // device error flag
   const int *perm_dev;    // internal -> original node id
+  // time functions of the Displacement_BC sets (as a kernel argument their
+  // 1.3 KB made up half of what a launch carries)
   // batched specimens (FP32C RNPBond): per-slice specimen id, per-specimen
-  // FP32 constants (Params32) and a global table of BC time functions
+  // FP32 constants (Params32)
   const int *slice_spec;
   const void *qtab;
   const BCTime *bct;
@@ -111,14 +118,14 @@ struct StepArgs {
 };
 
 // Launchers (return cudaError_t of the launch).
-cudaError_t launch_rnp_step_fp64(const StepParams &P, const DevPtrs &D, const BCTable &T,
+cudaError_t launch_rnp_step_fp64(const StepParams &P, const DevPtrs &D,
                                  const StepArgs &a, int decomp, cudaStream_t s);
-cudaError_t launch_rnp_step_fp32(const StepParams &P, const DevPtrs &D, const BCTable &T,
+cudaError_t launch_rnp_step_fp32(const StepParams &P, const DevPtrs &D,
                                  const StepArgs &a, int decomp, cudaStream_t s);
-cudaError_t launch_es_step_fp64(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                const StepArgs &a, int decomp, cudaStream_t s);
-cudaError_t launch_es_step_fp32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                                const StepArgs &a, int decomp, cudaStream_t s);
+cudaError_t launch_es_step_fp64(const StepParams &P, const DevPtrs &D,
+                                 const StepArgs &a, int decomp, cudaStream_t s);
+cudaError_t launch_es_step_fp32(const StepParams &P, const DevPtrs &D,
+                                 const StepArgs &a, int decomp, cudaStream_t s);
 // Lanes per node of the FP64 bond-store kernels, and their block size.
 int team64(int64_t n);
 constexpr int kTeamBlock = 64;
@@ -127,14 +134,14 @@ cudaError_t launch_rnp_store64(const StepParams &P, const DevPtrs &D, cudaStream
 cudaError_t launch_es_store64(const StepParams &P, const DevPtrs &D, cudaStream_t s);
 // Recompute the drift to u^{m+1} (and v^{m+1} for CD) from (u^m, v^m, f^m)
 // after the host replaced the state: the second half of the step epilogue.
-cudaError_t launch_drift(const StepParams &P, const DevPtrs &D, const BCTable &T, int cur,
+cudaError_t launch_drift(const StepParams &P, const DevPtrs &D, int cur,
                          double t_next, bool fp32, cudaStream_t s);
-cudaError_t launch_drift32(const StepParams &P, const DevPtrs &D, const BCTable &T, int cur,
+cudaError_t launch_drift32(const StepParams &P, const DevPtrs &D, int cur,
                            double t_next, cudaStream_t s);
 // Banded host step (FP32C, 2-D velocity Verlet): caller-order bands in and
 // out of staged copies of the caller's arrays, and the final commit.
-cudaError_t launch_pipe_in32(const StepParams &P, const DevPtrs &D, const BCTable &T,
-                             double t_next, int64_t o0, int64_t o1, const int *iperm,
+cudaError_t launch_pipe_in32(const StepParams &P, const DevPtrs &D,
+                                 double t_next, int64_t o0, int64_t o1, const int *iperm,
                              const double *hu, const double *hv, const double *hf, float4 *ua,
                              float4 *sv, float2 *sf, int *bad, cudaStream_t s);
 cudaError_t launch_pipe_out32(int64_t o0, int64_t o1, const int *list, const int *iperm,
@@ -145,6 +152,9 @@ cudaError_t launch_pipe_commit32(int64_t n, int64_t nbits, const int *bad, const
                                  const float4 *ub, const float4 *sv, const float2 *sf,
                                  float4 *u_now, float4 *u_next, float4 *v, float2 *f,
                                  uint32_t *bits, const uint32_t *bits_saved, cudaStream_t s);
+// out = flags with FLAG_RIM on the nodes that a no-fail bond ends at.
+cudaError_t mark_rim(int64_t n, const int64_t *rowptr, const int *cols, const uint8_t *flags,
+                     uint8_t *out, cudaStream_t s);
 cudaError_t launch_es_setup(const StepParams &P, const DevPtrs &D, double *mw, cudaStream_t s);
 cudaError_t launch_es_minv32(const double *mw, float *minv, int64_t n, cudaStream_t s);
 cudaError_t launch_damage(const StepParams &P, const DevPtrs &D, int cur, bool fp32,

@@ -7,34 +7,10 @@
 
 namespace nlm {
 
-// Time part of FLoading::apply (fLoading.cpp:246-266), applied as
-// fmax = (spatial * g(t)) * time_params[0].
-__device__ double fload_time(const BCTime &T, double fmax, double time) {
-  switch (T.fn) {
-    case NLM_TFN_LINEAR: fmax = fmax * time; break;
-    case NLM_TFN_LINEAR_STEP: {
-      const double x1 = T.p[1], x2 = T.p[2];
-      const double period = floor(time / (x1 + x2));
-      const double g = dLT(time, period * (x1 + x2) + x1) ? time - period * x2 : (period + 1.) * x1;
-      fmax = fmax * g;
-    } break;
-    case NLM_TFN_LINEAR_SLOW_FAST:
-      fmax = dGT(time, T.p[1]) ? fmax * (T.p[3] * time) : fmax * (T.p[2] * time);
-      break;
-    case NLM_TFN_SIN: fmax = fmax * sin((M_PI * T.p[1]) * time); break;
-    default: break;
-  }
-  return fmax * T.p[0];
-}
-
-
-// time: the load time, or tdev[0] when tdev is set (graph replay).
 __global__ void k_fbc_apply(int64_t nf, int S, const int *nodes, const int *iptr,
-                            const FBCItem *items, BCTable T, double time, double *fext,
-                            const double *tdev) {
+                            const FBCItem *items, BCTable T, double time, double *fext) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= nf) return;
-  if (tdev) time = tdev[0];
   double fe[3] = {0., 0., 0.};
   for (int k = iptr[t]; k < iptr[t + 1]; k++) {
     const FBCItem it = items[k];
@@ -184,6 +160,23 @@ __global__ void k_count_bits(int64_t n, int nwords, int64_t npad, const uint32_t
   int c = 0;
   for (int w = 0; w < nwords; w++) c += __popc(bits[(int64_t)w * npad + i]);
   if (c) atomicAdd(out, (unsigned long long)c);
+}
+
+__global__ void k_mark_rim(int64_t n, const int64_t *rowptr, const int *cols,
+                           const uint8_t *flags, uint8_t *out) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint8_t f = flags[i];
+  bool rim = f & FLAG_NOFAIL;
+  for (int64_t k = rowptr[i]; k < rowptr[i + 1] && !rim; k++) rim = flags[cols[k]] & FLAG_NOFAIL;
+  out[i] = rim ? f | FLAG_RIM : f;
+}
+
+cudaError_t mark_rim(int64_t n, const int64_t *rowptr, const int *cols, const uint8_t *flags,
+                     uint8_t *out, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  k_mark_rim<<<nblk(n, 256), 256, 0, s>>>(n, rowptr, cols, flags, out);
+  return cudaGetLastError();
 }
 
 }  // namespace nlm

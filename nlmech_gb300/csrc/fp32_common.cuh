@@ -290,10 +290,10 @@ __device__ __forceinline__ void st_pair(float4 *p, int64_t j, const df v[3]) {
 // Prescribed (du, dv) of one dof as double-float pairs.  Kept out of line:
 // only nodes with prescribed dofs call it, and inlined, its FP64 time
 // functions were if-converted into the path of every node.
-static __device__ __noinline__ void bc_df(const DevPtrs &D, const BCTable &T, int ref, int c, double t,
+static __device__ __noinline__ void bc_df(const DevPtrs &D, int ref, int c, double t,
                                    df &u, df &v) {
   double du, dv;
-  bc_dof(D, T, ref, c, t, du, dv);
+  bc_dof(D, ref, c, t, du, dv);
   u = df_from_double(du);
   v = df_from_double(dv);
 }
@@ -307,18 +307,18 @@ struct F3 {
   float c[3];
 };
 template <int DIM>
-static __device__ __noinline__ F3 fext_add32(const DevPtrs &D, int64_t i, F3 f) {
+static __device__ __noinline__ F3 fext_add32(const DevPtrs &D, int64_t i, double t, F3 f) {
   double fe[3];
-  ld_node<DIM>(D.fext, i, fe);
+  ext_force(D, i, t, fe);
   for (int c = 0; c < DIM; c++) f.c[c] = (float)(fe[c] + (double)f.c[c]);
   return f;
 }
 
 // FP32C integrator epilogue (same phase structure as integrate_node64).
-template <int DIM, int SCHEME>
+// LOADS: the model may have Force_BC nodes (a batch has none).
+template <int DIM, int SCHEME, bool LOADS = true>
 __device__ __forceinline__ void integrate_node32(const StepParams &P, const Params32 &Q,
-                                                 const DevPtrs &D, const BCTable &T,
-                                                 const StepArgs &A, int64_t i, uint8_t fl,
+                                                 const DevPtrs &D, const StepArgs &A, int64_t i, uint8_t fl,
                                                  const float uih[3], const float uil[3],
                                                  const float fint[3],
                                                  const float4 *vpre = nullptr,
@@ -326,8 +326,8 @@ __device__ __forceinline__ void integrate_node32(const StepParams &P, const Para
   // vpre, fpre (2-D): the node's velocity pair and previous force, already
   // staged in shared memory by the caller
   float f[3] = {fint[0], fint[1], fint[2]};
-  if (fl & FLAG_FBC) {
-    const F3 r = fext_add32<DIM>(D, i, F3{{fint[0], fint[1], fint[2]}});
+  if (LOADS && (fl & FLAG_FBC)) {
+    const F3 r = fext_add32<DIM>(D, i, t_now_of(A), F3{{fint[0], fint[1], fint[2]}});
     for (int c = 0; c < 3; c++) f[c] = r.c[c];
   }
   const int ref = (fl & 7) ? D.bcref[i] : -1;
@@ -370,12 +370,12 @@ __device__ __forceinline__ void integrate_node32(const StepParams &P, const Para
       } else {
         df du, dv;
         if (!FIRST) {
-          bc_df(D, T, ref, c, t_now, du, dv);
+          bc_df(D, ref, c, t_now, du, dv);
           vn[c] = dv;
         } else {
           vn[c] = v;
         }
-        bc_df(D, T, ref, c, t_next, du, dv);
+        bc_df(D, ref, c, t_next, du, dv);
         un[c] = du;
       }
     }
@@ -395,7 +395,7 @@ __device__ __forceinline__ void integrate_node32(const StepParams &P, const Para
         un[c] = df_add(u, inc);
         vn[c] = df_mul_c(df_sub(un[c], u), Q.idt_hi, Q.idt_lo);
       } else {
-        bc_df(D, T, ref, c, t_next, un[c], vn[c]);
+        bc_df(D, ref, c, t_next, un[c], vn[c]);
       }
     }
     st_pair<DIM>(D.v32[1 - A.cur], i, vn);

@@ -336,18 +336,17 @@ int step_host_banded(nlm_fd *h, double *u, double *v, double *f) {
   NLM_CUDA(cudaMemsetAsync(h->bad_input, 0, sizeof(int), s));
   NLM_CUDA(cudaMemcpyAsync(h->pipe_bits, h->D.bits, sizeof(uint32_t) * nbits,
                            cudaMemcpyDeviceToDevice, s));
-  if (int rc = apply_fbc(h, tm)) return rc;
   for (int k = 0; k < K; k++) {
     const int64_t o0 = bd[k], o1 = bd[k + 1];
     if (k + 2 < K)
       if (int rc = copy_in(k + 2)) return rc;
     NLM_CUDA(cudaStreamWaitEvent(s, h->pipe_ev[2 * k], 0));
-    NLM_CUDA(launch_pipe_in32(h->P, Dp, h->T, tm, o0, o1, h->iperm, in_u, in_v, in_f, h->pipe_ua,
+    NLM_CUDA(launch_pipe_in32(h->P, Dp, tm, o0, o1, h->iperm, in_u, in_v, in_f, h->pipe_ua,
                               h->pipe_v, h->pipe_f, h->bad_input, s));
     const int nk = h->pipe_toff[k + 1] - h->pipe_toff[k];
     if (nk > 0) {
       StepArgs a{c, false, tm, tm + h->dt, nullptr, 0, n, h->pipe_tiles + h->pipe_toff[k], nk};
-      const cudaError_t e = launch_rnp_step_fp32(h->P, Dp, h->T, a, h->decomp, s);
+      const cudaError_t e = launch_rnp_step_fp32(h->P, Dp, a, h->decomp, s);
       if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
     }
     for (int b : h->pipe_out[k]) {
@@ -430,7 +429,7 @@ int step_host_in_place(nlm_fd *h, double *u, double *v, double *f, int64_t nstep
   NLM_CUDA(cudaMemcpyAsync(du, su, bu, cudaMemcpyDeviceToDevice, s));
   NLM_CUDA(cudaMemcpyAsync(dv, sv, bu, cudaMemcpyDeviceToDevice, s));
   NLM_CUDA(cudaMemcpyAsync(df_, sf, bf, cudaMemcpyDeviceToDevice, s));
-  cudaError_t e = launch_drift(h->P, h->D, h->T, h->cur, h->time + h->dt, fp32, s);
+  cudaError_t e = launch_drift(h->P, h->D, h->cur, h->time + h->dt, fp32, s);
   if (e != cudaSuccess) return cuda_fail(e, "drift kernel");
   int rc = do_run(h, nsteps);
   if (rc) return rc;
@@ -527,7 +526,7 @@ int nlm_fd_step_host(nlm_fd *h, double *u, double *v, double *f, int64_t nsteps)
     k_scatter_vec<<<g, 256, 0, s>>>(n, h->S, h->dim, P, sf, h->D.f64);
   }
   NLM_CUDA(cudaGetLastError());
-  cudaError_t e = launch_drift(h->P, h->D, h->T, h->cur, h->time + h->dt, fp32, s);
+  cudaError_t e = launch_drift(h->P, h->D, h->cur, h->time + h->dt, fp32, s);
   if (e != cudaSuccess) return cuda_fail(e, "drift kernel");
   int rc = do_run(h, nsteps);
   if (rc) return rc;

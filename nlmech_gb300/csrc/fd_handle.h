@@ -247,6 +247,7 @@ int rnp_constants(const nlm_material &m, int dim, double delta, StepParams &P);
 int lattice_relabel(NeighborBuild &nb, int dim, int S, double mesh_h, double delta,
                     cudaStream_t s, std::vector<uint8_t> &lres);
 int create_model(const nlm_fd_desc *d, nlm_fd **out, bool explicit_steps);
+int build_bond_store64(nlm_fd *h);
 int launch_step(nlm_fd *h, const StepArgs &a0);
 int apply_fbc(nlm_fd *h, double t);
 int apply_bc(nlm_fd *h, double t);

@@ -134,6 +134,10 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
   }
   q->prm = *prm;
   nlm_fd *h = q->fd;
+  if ((rc = build_bond_store64(h))) {
+    delete q;
+    return rc;
+  }
   const int64_t n = h->n, m = (int64_t)h->dim * n, nnz = h->nnz;
   const int NB = h->dim == 2 ? 3 : 6;
   cudaError_t e = cudaSuccess;

@@ -994,17 +994,16 @@ int create_model(const nlm_fd_desc *d, nlm_fd **out, bool explicit_steps) {
     TRY(cudaMemcpyAsync(h->fbc_nodes, fnodes.data(), sizeof(int) * fnodes.size(), cudaMemcpyHostToDevice, s));
     TRY(cudaMemcpyAsync(h->fbc_iptr, fptr.data(), sizeof(int) * fptr.size(), cudaMemcpyHostToDevice, s));
     TRY(cudaMemcpyAsync(h->fbc_items, fits.data(), sizeof(FBCItem) * fits.size(), cudaMemcpyHostToDevice, s));
-    std::vector<int> fref(n, -1);
-    for (size_t k = 0; k < fnodes.size(); k++) fref[fnodes[k]] = (int)k;
-    int *dref;
+    std::vector<int2> fref(n, make_int2(0, 0));
+    for (size_t k = 0; k < fnodes.size(); k++) fref[fnodes[k]] = make_int2(fptr[k], fptr[k + 1]);
+    int2 *dref;
     BCTime *dt;
     TRY(h->alloc(&dref, n));
     TRY(h->alloc(&dt, kMaxBCSets));
-    TRY(cudaMemcpyAsync(dref, fref.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    TRY(cudaMemcpyAsync(dref, fref.data(), sizeof(int2) * n, cudaMemcpyHostToDevice, s));
     TRY(cudaMemcpyAsync(dt, h->FT.t, sizeof(BCTime) * kMaxBCSets, cudaMemcpyHostToDevice, s));
     TRY(cudaStreamSynchronize(s));
     D.fbc_ref = dref;
-    D.fbc_iptr = h->fbc_iptr;
     D.fbc_items = h->fbc_items;
     D.fbc_t = dt;
   }

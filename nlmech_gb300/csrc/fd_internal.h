@@ -21,8 +21,7 @@ struct DevPtrs {
   const BCEntry *bce;
   const double *fext;   // S doubles per node, valid where FLAG_FBC is set (the
                         // quasi-static models; a time step evaluates the loads)
-  const int *fbc_ref;   // node -> its entry of fbc_iptr (-1: none)
-  const int *fbc_iptr;  // items of an entry: fbc_iptr[e] .. fbc_iptr[e + 1]
+  const int2 *fbc_ref;  // node -> its items [x, y)
   const FBCItem *fbc_items;
   const BCTime *fbc_t;  // time functions by set
   // topology

@@ -1354,6 +1354,12 @@ static cudaError_t qs_cg32_res(const StepParams &P, const DevPtrs &D, QSWork &W,
   e = cudaLaunchCooperativeKernel(
       P.dim == 2 ? (const void *)k_cg32_res<2> : (const void *)k_cg32_res<3>, A.blocks,
       kResThreads, args, W.res_smem, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    // fewer SMs to be had than at creation: the two-launch form
+    cudaGetLastError();
+    W.kr.blocks = 0;
+    return cudaSuccess;
+  }
   double r[4] = {};
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(r, A.res, sizeof(r), cudaMemcpyDeviceToHost, s);
@@ -1482,7 +1488,7 @@ cudaError_t qs_cg(const StepParams &P, const DevPtrs &D, QSWork &W, const double
         W.kr.blocks = 0;  // the two-launch form from now on
       }
     }
-    if (e == cudaSuccess && (W.kr.blocks == 0 || status != 0))
+    if (e == cudaSuccess && W.kr.blocks == 0)
       e = qs_cg32(P, D, W, rhs, dx, tol, cap, check_every, &it32, &conv, s);
     if (e != cudaSuccess || conv || max_iters <= kCg32Cap) {
       *iters = it32;

@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(128)
 // operations each (div_by), and the break test is an integer comparison with
 // a bound below the extension at s_c.  The remaining operations are those of
 // k_es_dil64 and k_es_force64 in their order: the same bits.  31 x 29 x 27
-// block: 1596 us per step with those kernels, 371 us here (the FP64 pipe 81 %
-// busy, about 85 instructions per bond); 60^3 cube: 3165 us.
+// block: 1596 us per step with those kernels, 371 us here (the FP64 pipe 79 and
+// 84 % busy, 80 instructions per bond); 60^3 cube: 3165 us.
 
 template <int DIM>
 __global__ void k_es_store64(const StepParams P, const DevPtrs D, double2 *bx, double *bv, int *bt,

@@ -165,7 +165,7 @@ __global__ void k_rnp64_store(const StepParams P, const DevPtrs D, double2 *bd, 
 // their contributions are added in row order.  Four bonds per lane take 139
 // registers and were slower (189 against 146 us), so are blocks of 128 (159).
 // 320 x 250 plate, horizon 3h: 605 us per step with k_rnp64_thread, 146 us
-// here, 33 FP64 instructions per bond, the FP64 pipe 85 % busy: the bound.
+// here, 33 FP64 instructions per bond, the FP64 pipe 82 % busy: the bound.
 template <int DIM, int SCHEME, bool FIRST, int G>
 __global__ void __launch_bounds__(128)
     k_rnp64_bond(const StepParams P, const double inv_invF, const DevPtrs D, const StepArgs A) {

@@ -453,7 +453,7 @@ int autotune(nlm_fd *h) {
   int pick = NLM_DECOMP_THREAD;
   StepArgs sa{0, false, h->time, h->time + h->dt, nullptr, 0, h->n};
   sa.pdl = true;  // as the steps of a run are launched
-  const int reps = n < 100000 ? 25 : 5;  // 5 launches of 7 us differ by more than the candidates
+  const int reps = n < 100000 ? 12 : 5;  // 5 launches of 7 us differ by more than the candidates
   for (int c : cands) {
     auto launch = [&]() {
       return rnp ? launch_rnp_step_fp32(h->P, D, sa, c, s)

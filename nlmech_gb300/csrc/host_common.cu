@@ -26,14 +26,29 @@ int fail(int code, const std::string &msg) {
 
 const char *last_error() { return g_err.c_str(); }
 
+// Bytes of [b, e) (page bounds) that are not resident; as if all were where the
+// kernel does not say.
+static size_t missing_bytes(uintptr_t b, uintptr_t e, size_t page) {
+  unsigned char in[1024];
+  size_t out = 0;
+  for (; b < e; b += sizeof(in) * page) {
+    const size_t len = std::min<size_t>(e - b, sizeof(in) * page);
+    if (mincore((void *)b, len, in) != 0) return out + (e - b);
+    for (size_t k = 0; k < len / page; k++)
+      if (!(in[k] & 1)) out += page;
+  }
+  return out;
+}
+
 // Pages of a fresh allocation that a device copy meets first are made resident
 // one fault at a time: 84 MB took 30 ms to receive (2.8 GB/s), prefaulted before
 // 0.7 ms.  madvise(MADV_POPULATE_WRITE) faults them for writing and keeps their
 // contents: 2.7 ms for the 84 MB, 1.5 ms by two threads (1.5 by four); touching
 // them by reading and writing back costs 30 ms, the read maps the zero page
-// first.  Resident pages cost microseconds.  Where the call is not to be had the
-// copy faults the pages as before.  Small arrays usually lie in memory the
-// process has used.
+// first.  Arrays that the caller keeps are resident, and the second thread cost
+// every read-back into them 100 us (6 MB: 202 us without, 315 with it), so the
+// kernel is asked first (mincore, 4 us for 72 MB) and little that is missing is
+// left to the copy, as is all of it where a call is not to be had.
 void prefault(std::initializer_list<std::pair<void *, size_t>> arrays) {
   constexpr size_t kMin = 4 << 20;
   constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, Linux 5.14
@@ -43,6 +58,12 @@ void prefault(std::initializer_list<std::pair<void *, size_t>> arrays) {
   size_t total = 0;
   for (auto &a : arrays)
     if (a.first) total += a.second;
+  if (total < kMin) return;
+  total = 0;
+  for (auto &a : arrays)
+    if (a.first && a.second)
+      total += missing_bytes((uintptr_t)a.first & ~mask,
+                             ((uintptr_t)a.first + a.second + mask) & ~mask, (size_t)ps);
   if (total < kMin) return;
   auto half = [&](int w) {
     for (auto &a : arrays) {

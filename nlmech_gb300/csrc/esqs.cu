@@ -311,7 +311,11 @@ __global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *rows, int *ocol
 //   shadow: alpha, s = r - alpha v, t = J s, partials of s.s, t.s, t.t, rhat.s
 //           and rhat.t
 // r.r and rhat.r follow from shadow's sums (r = s - omega t with omega =
-// t.s / t.t), which saves the third launch a separate sum over r would need.  r,
+// t.s / t.t), which saves the third launch a separate sum over r would need,
+// unless they cancel: where r.r comes out below kBiCancel s.s (a half step that
+// all but solves the system; its last bits would decide on convergence) that dir
+// stops after forming r and sums it, shadow passes, and the next dir goes on from
+// those sums, one pair of launches more.  r,
 // p and s of a neighbour are formed where the product reads them, partial sums
 // are added by one warp of every block of the next launch in one fixed order
 // while the others fetch their blocks of J, and a launch after convergence does
@@ -323,6 +327,7 @@ __global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *rows, int *ocol
 
 constexpr int kBiThreads = 64;
 constexpr int kBiTeam = 8;  // lanes per row of J
+constexpr double kBiCancel = 0x1p-10;  // r.r by difference: good to 2^-42 or better
 
 // Totals of N partial arrays of gridDim.x entries each, in one fixed order
 // (one warp; lane 0 ends with them).
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_init(const BiArgs B, const do
   }
   sum[3] = sum[0];
   bi_partials<5>(sum, B.part2);
-  if (blockIdx.x == 0 && threadIdx.x == 0) B.sc[2] = BiScal{1., 0., 0., 0., 0., 0, 0};
+  if (blockIdx.x == 0 && threadIdx.x == 0) B.sc[2] = BiScal{1., 0., 0., 0., 0., BI_RUN, 0, 0};
 }
 
 // A team's share of row i of J (block b = g, g + 8, ...): the first PF blocks
@@ -431,55 +436,80 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x < 32) {
     BiScal sc = B.sc[2 + ((k ^ 1) & 1)];
+    // the last dir launch updated x and r and summed r.r and rhat.r
+    const bool summed = sc.done == BI_SUM;
     double t[5];  // s.s, t.s, t.t, rhat.s, rhat.t
-    bi_totals<5>(B.part2, t);
+    if (summed)
+      bi_totals<2>(B.part3, t);
+    else
+      bi_totals<5>(B.part2, t);
     if (threadIdx.x == 0) {
-      if (!sc.done) {
+      if (sc.done == BI_RUN || summed) {
         const double rho = sc.rho;
+        bool end, cancel = false;
         if (sc.iters == 0) {
           sc.stop2 = B.tol * B.tol * t[0];
           sc.rho = t[3];
           sc.beta = sc.omega = 0.;
-          sc.done = t[0] == 0.;
+          end = t[0] == 0.;
         } else {
-          const bool half = t[0] <= sc.stop2 || t[2] == 0.;
-          sc.omega = half ? 0. : t[1] / t[2];
-          sc.rho = __fma_rn(-sc.omega, t[4], t[3]);
-          sc.beta = (sc.rho / rho) * (sc.alpha / sc.omega);
-          sc.done = half || __fma_rn(-sc.omega, t[1], t[0]) <= sc.stop2 || sc.omega == 0. ||
-                    sc.iters >= B.max_iters;
+          double rr = t[0];
+          bool half = false;
+          if (summed) {
+            sc.rho = t[1];
+          } else {
+            half = t[0] <= sc.stop2 || t[2] == 0.;
+            sc.omega = half ? 0. : t[1] / t[2];
+            rr = __fma_rn(-sc.omega, t[1], t[0]);
+            cancel = !half && sc.omega != 0. && rr < kBiCancel * t[0];
+            if (!cancel) sc.rho = __fma_rn(-sc.omega, t[4], t[3]);
+          }
+          if (!cancel) sc.beta = (sc.rho / rho) * (sc.alpha / sc.omega);
+          end = half || rr <= sc.stop2 || sc.omega == 0. || sc.iters >= B.max_iters;
         }
-        if (!sc.done) {
-          sc.iters++;
-          if (sc.rho == 0.) sc.done = 1;  // breakdown: keep the iterate
+        if (cancel) {
+          sc.done = BI_SUM;
+        } else {
+          if (!end) {
+            sc.iters++;
+            end = sc.rho == 0.;  // breakdown: keep the iterate
+          }
+          // the solve's last x update is still due in this launch
+          sc.done = end ? BI_LAST : BI_RUN;
         }
-        // the solve's last x update is still due in this launch
-        sc.done = sc.done ? 2 : 0;
       } else {
-        sc.done = 1;
+        sc.done = BI_DONE;
       }
+      sc.moved = summed;
       s_sc = sc;
       if (blockIdx.x == 0) B.sc[k & 1] = sc;
     }
   }
   __syncthreads();
   const BiScal sc = s_sc;
-  if (sc.done == 1) return;
+  if (sc.done == BI_DONE) return;
   const double *po = B.p[(k ^ 1) & 1], *vo = B.v[(k ^ 1) & 1];
   double *pn = B.p[k & 1], *vn = B.v[k & 1];
   const double bo = -sc.beta * sc.omega;
-  double rv[1] = {};
+  double rv[2] = {};
   for (int64_t i0 = blockIdx.x * kBiRows; i0 < B.n; i0 += gridDim.x * kBiRows) {
     const int64_t it = i0 + threadIdx.x / kBiTeam;
     if (it != first_row) row.fetch(B, min(it, B.n - 1), g);
     const int64_t i = row.i;
     const bool own = g == 0 && it < B.n;
-    if (own)
+    if (own && !sc.moved)
       for (int d = 0; d < MD; d++) {
         const int64_t q = S * i + d;
-        const double s = B.s[q];
+        const double s = B.s[q], r = __fma_rn(-sc.omega, B.t[q], s);
         B.x[q] = __fma_rn(sc.omega, s, __fma_rn(sc.alpha, po[q], B.x[q]));
-        B.r[q] = __fma_rn(-sc.omega, B.t[q], s);
+        B.r[q] = r;
+        if (sc.done == BI_SUM) {
+          // p and v for the next launch, which reads this one's slots
+          pn[q] = po[q];
+          vn[q] = vo[q];
+          rv[0] = __fma_rn(r, r, rv[0]);
+          rv[1] = __fma_rn(B.rhat[q], r, rv[1]);
+        }
       }
     if (sc.done) continue;
     auto val = [&](int64_t j, double *y) {
@@ -504,7 +534,10 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_dir(const BiArgs B, int k) {
       }
     }
   }
-  if (!sc.done) bi_partials<1>(rv, B.part1);
+  if (sc.done == BI_SUM)
+    bi_partials<2>(rv, B.part3);
+  else if (!sc.done)
+    bi_partials<1>(rv, B.part1);
 }
 
 template <int MD>
@@ -524,7 +557,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_shadow(const BiArgs B, int k)
     if (threadIdx.x == 0) {
       if (!sc.done) {
         if (t[0] == 0.)
-          sc.done = 1;  // breakdown: keep the iterate
+          sc.done = BI_DONE;  // breakdown: keep the iterate
         else
           sc.alpha = sc.rho / t[0];
       }
@@ -683,7 +716,8 @@ cudaError_t esqs_bicgstab(const BiArgs &B, cudaGraphExec_t graph, const double *
   k_bi_init<<<B.blocks, kBiThreads, 0, s>>>(B, rhs);
   cudaError_t e = cudaGetLastError();
   BiScal st{};
-  while (e == cudaSuccess && !st.done) {  // max_iters ends it on the device
+  // max_iters ends it on the device
+  while (e == cudaSuccess && (st.done == BI_RUN || st.done == BI_SUM)) {
     e = cudaGraphLaunch(graph, s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(&st, B.sc + 2, sizeof(st), cudaMemcpyDeviceToHost, s);

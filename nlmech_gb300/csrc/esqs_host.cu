@@ -114,6 +114,7 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
     if (e == cudaSuccess) e = q->alloc(ptr, q->m);
   if (e == cudaSuccess) e = q->alloc(&bi.part1, kBiParts);
   if (e == cudaSuccess) e = q->alloc(&bi.part2, 5 * kBiParts);
+  if (e == cudaSuccess) e = q->alloc(&bi.part3, 2 * kBiParts);
   if (e == cudaSuccess) e = q->alloc(&bi.sc, 4);
   const size_t md = (size_t)q->mdim;
   if (e == cudaSuccess) e = q->alloc(&q->J, md * md * q->nblocks);

@@ -31,7 +31,11 @@ cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim
 struct BiScal {
   double rho, alpha, omega, beta, stop2;
   int done, iters;
+  int moved;                // x and r are those of this iteration's end already
 };
+// done: the solve goes on, is over, ends with the x update of this dir launch, or
+// sums r.r and rhat.r afresh in it
+enum { BI_RUN = 0, BI_DONE = 1, BI_LAST = 2, BI_SUM = 3 };
 constexpr int kBiParts = 1216;  // most blocks of a launch (8 per SM)
 struct BiArgs {
   int64_t n, m;             // nodes, entries of a vector (S per node)
@@ -40,7 +44,7 @@ struct BiArgs {
   const int *cols;
   const double *J;
   double *r, *rhat, *p[2], *v[2], *s, *t, *x;
-  double *part1, *part2;    // kBiParts and 5 kBiParts doubles
+  double *part1, *part2, *part3;  // kBiParts, 5 kBiParts and 2 kBiParts doubles
   int blocks;
   BiScal *sc;               // 4
   double tol;               // ||r|| <= tol ||rhs||

@@ -441,7 +441,9 @@ typedef struct nlm_qs_params {
                           2-D bonds), else in two launches per iteration;
                           200 x 200 plate: 7 us per iteration against 27
                           1: the same, but a wait of that launch that runs out
-                          is an error instead of a change to two launches   */
+                          is an error instead of a change to two launches
+                          2: two launches per iteration always
+                          (nlm_qs_krylov_form tells which form is in use)    */
   double wait_limit_s; /* bound of each grid-wide wait of that launch
                           (<= 0: 1 s); a wait that runs out ends the launch;
                           with krylov_launch = 1 the load step then fails with
@@ -486,6 +488,10 @@ int nlm_qs_get_state(nlm_qs *q, double *u);
 int nlm_qs_get_bond_state(nlm_qs *q, uint8_t *broken);
 int nlm_qs_damage(nlm_qs *q, float *phi, float *Z);
 int nlm_qs_num_bonds(const nlm_qs *q, int64_t *nnz);
+/* The form that FP32 Krylov solves of this handle take from here on: 1 one
+ * cooperative launch per solve, 2 two launches per iteration (asked for, or the
+ * tangent does not fit, or, with krylov_launch = 0, a wait has run out). */
+int nlm_qs_krylov_form(const nlm_qs *q, int *form);
 
 /* ---- quasi-static ElasticState (the reference's QuasiStaticModel) -------
  * QuasiStaticModel<ElasticState> (src/model/quasistatic/QuasiStaticModel.cpp,

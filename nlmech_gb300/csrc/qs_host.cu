@@ -158,7 +158,7 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
   if (e == cudaSuccess) e = q->alloc(&q->W.sc, 8);
   if (e == cudaSuccess) e = q->alloc(&q->W.blk, (size_t)NB * (nnz + 1));
   if (e == cudaSuccess) e = q->alloc(&q->W.dblk, (size_t)NB * n);
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && (prm->krylov_launch == 0 || prm->krylov_launch == 1))
     e = qs_res_setup(h->P, h->D, h->rowptr.data(), q->W,
                      [&](void **p, size_t bytes) { return q->alloc((char **)p, bytes); },
                      h->stream);
@@ -287,6 +287,12 @@ int nlm_qs_damage(nlm_qs *q, float *phi, float *Z) {
 int nlm_qs_num_bonds(const nlm_qs *q, int64_t *nnz) {
   if (!q) return fail(NLM_ERR_INVALID, "null handle");
   return nlm_fd_num_bonds(q->fd, nnz);
+}
+
+int nlm_qs_krylov_form(const nlm_qs *q, int *form) {
+  if (!q || !form) return fail(NLM_ERR_INVALID, "null argument");
+  *form = q->W.kr.blocks > 0 ? 1 : 2;
+  return NLM_OK;
 }
 
 }  // extern "C"

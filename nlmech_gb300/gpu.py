@@ -339,7 +339,8 @@ def qs_params(max_newton=30, tol=1e-8, lin_max_iters=20000, lin_tol=1e-4, break_
     """nlm_qs_params; krylov_launch 0: the FP32 Krylov solve in one
     cooperative launch where the tangent fits on the SMs, else (or after a wait
     of that launch ran out) in two launches per iteration, 1: a wait that runs
-    out (wait_limit_s) is an error instead; barrier_extra > 0 only to test the
+    out (wait_limit_s) is an error instead, 2: two launches per iteration
+    always (QSModel.krylov_form tells); barrier_extra > 0 only to test the
     bounded wait; lin_tol_gamma > 0 loosens the Krylov tolerance of a Newton
     iteration whose residual is already near the target."""
     return abi.QSParams(max_newton, tol, lin_max_iters, lin_tol, int(break_bonds),
@@ -390,6 +391,13 @@ class QSModel:
     def nnz(self):
         v = C.c_int64()
         _check(load().nlm_qs_num_bonds(self.h, C.byref(v)))
+        return v.value
+
+    def krylov_form(self):
+        """The form of the FP32 Krylov solves from here on: 1 one cooperative
+        launch per solve, 2 two launches per iteration."""
+        v = C.c_int()
+        _check(load().nlm_qs_krylov_form(self.h, C.byref(v)))
         return v.value
 
     def bond_state(self):

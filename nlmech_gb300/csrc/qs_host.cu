@@ -134,10 +134,6 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
   }
   q->prm = *prm;
   nlm_fd *h = q->fd;
-  if ((rc = build_bond_store64(h))) {
-    delete q;
-    return rc;
-  }
   const int64_t n = h->n, m = (int64_t)h->dim * n, nnz = h->nnz;
   const int NB = h->dim == 2 ? 3 : 6;
   cudaError_t e = cudaSuccess;
@@ -162,6 +158,10 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
     e = qs_res_setup(h->P, h->D, h->rowptr.data(), q->W,
                      [&](void **p, size_t bytes) { return q->alloc((char **)p, bytes); },
                      h->stream);
+  if (e == cudaErrorMemoryAllocation && q->W.kr.blocks == 0 && q->W.dblk) {
+    cudaGetLastError();  // no room for its layout: two launches per iteration
+    e = cudaSuccess;
+  }
   q->W.res_only = prm->krylov_launch == 1;
   q->W.kr.extra = std::max(0, std::min(prm->barrier_extra, 64));
   q->W.kr.wait_ns =
@@ -172,6 +172,12 @@ int nlm_qs_create(const nlm_fd_desc *desc, const nlm_qs_params *prm, nlm_qs **ou
   if (e != cudaSuccess) {
     delete q;
     return cuda_fail(e, "qs buffers");
+  }
+  // last, from what the buffers have left: taken first, it could leave a model
+  // without them that fits without it
+  if ((rc = build_bond_store64(h))) {
+    delete q;
+    return rc;
   }
   h->started = true;  // no explicit step-0 evaluation
   *out = q;

@@ -13,6 +13,9 @@ static thread_local std::string g_err;
 void set_error(const std::string &msg) { g_err = msg; }
 int cuda_fail(cudaError_t e, const char *what) {
   g_err = std::string(what) + ": " + cudaGetErrorString(e);
+  // reported here: left standing, a failed allocation was found by the launch
+  // check of the next call, which then failed for it
+  (void)cudaGetLastError();
   if (e == cudaErrorMemoryAllocation) return NLM_ERR_OOM;
   // the solvers' bounded grid-barrier waits report a wait that ran out so
   if (e == cudaErrorTimeout) return NLM_ERR_TIMEOUT;

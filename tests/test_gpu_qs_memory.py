@@ -44,3 +44,22 @@ def test_store_does_not_take_the_solvers_memory(gpu):
         torch.cuda.empty_cache()
     # the geometry recomputed instead of read: rounding, before the truncated solve
     assert abs(v - u).max() <= 1e-6 * abs(u).max()
+
+
+def test_a_failed_create_leaves_the_next_call_alone(gpu):
+    torch = pytest.importorskip("torch")
+    p = configs.qs_plate(300, h=5e-4, du=1e-8)
+    gpu.QSModel(p).close()
+    torch.empty(1, device="cuda")
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8,
+                         device="cuda")
+    try:
+        with pytest.raises(gpu.NLMError) as e:
+            gpu.QSModel(p)
+        assert e.value.code == 3  # NLM_ERR_OOM
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    q = gpu.QSModel(p)
+    assert q.load_step()["newton_iters"] > 0

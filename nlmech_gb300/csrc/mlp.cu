@@ -399,6 +399,17 @@ struct nlm_mlp {
     }
     return e;
   }
+  // alloc() in the place of what *p held (null: nothing), so that a handle keeps
+  // one set of buffers however its row counts grow; *p is null where it fails
+  template <class Tp>
+  cudaError_t realloc(Tp **p, size_t count) {
+    if (*p) {
+      allocs.erase(std::find(allocs.begin(), allocs.end(), (void *)*p));
+      cudaFree(*p);
+      *p = nullptr;
+    }
+    return alloc(p, count);
+  }
   ~nlm_mlp() {
     if (s) cudaStreamSynchronize(s);
     for (void *p : allocs) cudaFree(p);
@@ -418,18 +429,19 @@ cudaError_t ensure_cap(nlm_mlp *h, int64_t rows) {
   const int64_t cap = std::max<int64_t>(rows, 1024);
   cudaError_t e = cudaSuccess;
   const int L = h->nl + 1;
-  h->Z.assign(L, nullptr);
-  h->A.assign(L + 1, nullptr);
-  h->dZ.assign(L, nullptr);
-  e = h->alloc(&h->A[0], (size_t)cap * h->kin);
+  h->Z.resize(L, nullptr);
+  h->A.resize(L + 1, nullptr);
+  h->dZ.resize(L, nullptr);
+  h->cap = 0;  // until all of them are there
+  e = h->realloc(&h->A[0], (size_t)cap * h->kin);
   for (int l = 0; l < L && e == cudaSuccess; l++) {
-    e = h->alloc(&h->Z[l], (size_t)cap * h->dout[l]);
-    if (e == cudaSuccess) e = h->alloc(&h->A[l + 1], (size_t)cap * h->dout[l]);
-    if (e == cudaSuccess) e = h->alloc(&h->dZ[l], (size_t)cap * h->dout[l]);
+    e = h->realloc(&h->Z[l], (size_t)cap * h->dout[l]);
+    if (e == cudaSuccess) e = h->realloc(&h->A[l + 1], (size_t)cap * h->dout[l]);
+    if (e == cudaSuccess) e = h->realloc(&h->dZ[l], (size_t)cap * h->dout[l]);
   }
-  if (e == cudaSuccess) e = h->alloc(&h->xbuf, (size_t)cap * h->nin);
-  if (e == cudaSuccess) e = h->alloc(&h->tbuf, (size_t)cap * h->nout);
-  if (e == cudaSuccess) e = h->alloc(&h->ybuf, (size_t)cap * h->nout);
+  if (e == cudaSuccess) e = h->realloc(&h->xbuf, (size_t)cap * h->nin);
+  if (e == cudaSuccess) e = h->realloc(&h->tbuf, (size_t)cap * h->nout);
+  if (e == cudaSuccess) e = h->realloc(&h->ybuf, (size_t)cap * h->nout);
   if (e == cudaSuccess) h->cap = cap;
   return e;
 }
@@ -671,9 +683,11 @@ int nlm_mlp_forward(nlm_mlp *h, const float *x, int64_t rows, float *y) {
   if (!h || !x || !y || rows < 0) return fail2(NLM_ERR_INVALID, "bad arguments");
   if (rows == 0) return NLM_OK;
   if (rows > h->icap) {
-    const int64_t cap = std::max<int64_t>(rows, 1024);
-    NLM_CUDA(h->alloc(&h->ix, (size_t)cap * h->nin));
-    NLM_CUDA(h->alloc(&h->iy, (size_t)cap * h->nout));
+    // half as much again, so that slowly growing calls seldom allocate
+    const int64_t cap = std::max<int64_t>(std::max<int64_t>(rows, h->icap + h->icap / 2), 1024);
+    h->icap = 0;
+    NLM_CUDA(h->realloc(&h->ix, (size_t)cap * h->nin));
+    NLM_CUDA(h->realloc(&h->iy, (size_t)cap * h->nout));
     h->icap = cap;
   }
   NLM_CUDA(cudaMemcpyAsync(h->ix, x, sizeof(float) * rows * h->nin, cudaMemcpyHostToDevice, h->s));
@@ -714,9 +728,10 @@ int nlm_mlp_grad(nlm_mlp *h, const float *x, const float *t, int64_t rows, float
 int nlm_mlp_set_data(nlm_mlp *h, const float *x, const float *t, int64_t rows) {
   if (!h || !x || !t || rows <= 0) return fail2(NLM_ERR_INVALID, "bad arguments");
   if (rows > h->drows) {
-    NLM_CUDA(h->alloc(&h->dx, (size_t)rows * h->nin));
-    NLM_CUDA(h->alloc(&h->dy, (size_t)rows * h->nout));
-    NLM_CUDA(h->alloc(&h->didx, (size_t)rows));
+    h->drows = 0;
+    NLM_CUDA(h->realloc(&h->dx, (size_t)rows * h->nin));
+    NLM_CUDA(h->realloc(&h->dy, (size_t)rows * h->nout));
+    NLM_CUDA(h->realloc(&h->didx, (size_t)rows));
   }
   h->drows = rows;
   NLM_CUDA(cudaMemcpyAsync(h->dx, x, sizeof(float) * rows * h->nin, cudaMemcpyHostToDevice, h->s));

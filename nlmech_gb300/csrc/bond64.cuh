@@ -2,15 +2,14 @@
 // quasi-static residual in qs.cu).
 #pragma once
 
-#include "common.cuh"
-
 namespace nlm {
 
-// exp(x): the Taylor polynomial of degree 7 where |x| < 2^-5 (bonds below a
-// quarter of the critical strain; truncation 2^-55, last operation a fused
-// 1 + x q, so within 0.53 ulp), CUDA's exp() elsewhere.  The polynomial is 7
-// FP64 instructions against about 19.
-constexpr int kExpSmall = 0x3fa00000;  // high word of 2^-5
+// exp(x): the Taylor polynomial of degree 7 where |x| < 2^-6 (bonds below 0.18 of
+// the critical strain; truncation 2^-63, last operation a fused 1 + x q: within
+// 0.506 ulp, tests/test_exp_small.py), CUDA's exp() elsewhere.  Up to 2^-5 the
+// truncation of 2^-55 counts: 0.69 ulp below 0, where results lie under 1.  The
+// polynomial is 7 FP64 instructions against about 19.
+constexpr int kExpSmall = 0x3f900000;  // high word of 2^-6
 __device__ __forceinline__ double exp_small(double x) {
   double q = 1. / 5040.;
   q = __fma_rn(q, x, 1. / 720.);

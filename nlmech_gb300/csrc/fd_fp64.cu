@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(128)
 // geometry only (two square roots, four divisions, the volume factor).  The
 // bond store keeps those values (68 bytes per 2-D bond, read once per step in
 // 512-byte rows); every remaining operation is the reference's, rounded in
-// the same order, so the results are the same bits.
+// the same order, so the results are those of k_rnp64_thread bit for bit (both
+// take exp64, the series below a sixth of the critical strain).
 // b64_thr: the high word of the break threshold S_c(r), below which |S| cannot
 // break the bond (one integer comparison instead of FP64 ones); bit 31 marks a
 // bond of a no-fail node, whose threshold is that of infinity.

@@ -144,57 +144,82 @@ __global__ void k_esqs_residual(int64_t n, const uint8_t *flags, int mdim, const
 // Bound by latency at a few thousand rows.  40 x 36 plate, horizon 3h: a load
 // step with three Jacobians took 135 ms before and 89 ms with these kernels.
 
-// One thread per directed bond q = (i, j), mdim <= 3 components; per bond
-// B (mdim), H (mdim), g = dF_ij/dtheta_i (mdim) and A (mdim^2, row-major).
-template <int SD>
-__global__ void k_esqs_bonds(const StepParams P, const DevPtrs D, int mdim, const int *rows,
-                             int64_t nnz, const double *u, const double *theta, double eps,
-                             double *out) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= nnz) return;
-  const int64_t i = rows[q], j = D.cols[q];
-  double xi[3], ui[3], xj[3], uj[3], Y[3], Xl, e;
+// A warp per row i, a lane per bond q = (i, j): per bond B and H (MD doubles each)
+// go to bond, A (MD^2, row-major) to the place of the bond's block in J, and the
+// row's sums of B, g = dF_ij/dtheta_i and A, in one fixed order, to sums.  (With g
+// and A in bond as well and the sums in a launch of their own, the workspace of a
+// 3-D bond was 144 bytes beside the 72 of J, 48 now; same bits.)
+template <int SD, int MD>
+__global__ void __launch_bounds__(128)
+    k_esqs_bonds(const StepParams P, const DevPtrs D, const double *u, const double *theta,
+                 double eps, double *bond, double *sums, double *J) {
+  constexpr int R = 2 * MD, Q = 2 * MD + MD * MD, M2 = MD * MD;
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (i >= P.n) return;
+  const int lane = threadIdx.x & 31;
+  double xi[3], ui[3];
   ld_node<SD>(D.pos64, i, xi);
   ld_node_rw<SD>(u, i, ui);
-  ld_node<SD>(D.pos64, j, xj);
-  ld_node_rw<SD>(u, j, uj);
-  es_geom64<SD>(xi, ui, xj, uj, Y, Xl, e);
-  const double Yl = sqrt(Y[0] * Y[0] + Y[1] * Y[1] + Y[2] * Y[2]);
-  const double mi = D.mw64[i], mj = D.mw64[j], thi = theta[i], thj = theta[j];
-  const double wv = es_omega(P, Xl) * D.vol64[j];
-  const double cth = ((double)mdim / mi) * (mdim == 2 ? P.es_factor2D : 1.) * Xl * wv;
-  // dt/dtheta of both ends
-  double ai = 0., aj = 0.;
-  if (mdim == 2) {
-    const double2 ci = es_coef64<2>(P, mi), cj = es_coef64<2>(P, mj);
-    ai = (ci.x / 3. - ci.y) * Xl / 3.;
-    aj = (cj.x / 3. - cj.y) * Xl / 3.;
-  } else if (mdim == 3) {
-    const double2 ci = es_coef64<3>(P, mi), cj = es_coef64<3>(P, mj);
-    ai = (ci.x - (P.es_ref_compat ? 0. : ci.y)) * Xl / 3.;
-    aj = (cj.x - (P.es_ref_compat ? 0. : cj.y)) * Xl / 3.;
-  }
-  double *o = out + (int64_t)(3 * mdim + mdim * mdim) * q;
-  for (int d = 0; d < mdim; d++) {
-    const double f = Y[d] / Yl * wv;
-    o[mdim + d] = f * aj;
-    o[2 * mdim + d] = f * ai;
-  }
-  for (int rr = 0; rr < mdim; rr++) {
-    double F[2][3], E[2];
-    for (int w = 0; w < 2; w++) {
-      double um[3] = {uj[0], uj[1], uj[2]}, Z[3], Xm;
-      um[rr] = um[rr] + (w ? -eps : eps);
-      es_geom64<SD>(xi, ui, xj, um, Z, Xm, E[w]);
-      const double Zl = sqrt(Z[0] * Z[0] + Z[1] * Z[1] + Z[2] * Z[2]);
-      const double s =
-          (esqs_t(P, mdim, mi, thi, E[w], Xl) + esqs_t(P, mdim, mj, thj, E[w], Xl)) * wv;
-      for (int d = 0; d < 3; d++) F[w][d] = (Z[d] / Zl) * s;
+  const double mi = D.mw64[i], thi = theta[i];
+  double sum[Q] = {};
+  for (int64_t q = D.rowptr[i] + lane; q < D.rowptr[i + 1]; q += 32) {
+    const int64_t j = D.cols[q];
+    double xj[3], uj[3], Y[3], Xl, e;
+    ld_node<SD>(D.pos64, j, xj);
+    ld_node_rw<SD>(u, j, uj);
+    es_geom64<SD>(xi, ui, xj, uj, Y, Xl, e);
+    const double Yl = sqrt(Y[0] * Y[0] + Y[1] * Y[1] + Y[2] * Y[2]);
+    const double mj = D.mw64[j], thj = theta[j];
+    const double wv = es_omega(P, Xl) * D.vol64[j];
+    const double cth = ((double)MD / mi) * (MD == 2 ? P.es_factor2D : 1.) * Xl * wv;
+    // dt/dtheta of both ends
+    double ai = 0., aj = 0.;
+    if (MD == 2) {
+      const double2 ci = es_coef64<2>(P, mi), cj = es_coef64<2>(P, mj);
+      ai = (ci.x / 3. - ci.y) * Xl / 3.;
+      aj = (cj.x / 3. - cj.y) * Xl / 3.;
+    } else if (MD == 3) {
+      const double2 ci = es_coef64<3>(P, mi), cj = es_coef64<3>(P, mj);
+      ai = (ci.x - (P.es_ref_compat ? 0. : ci.y)) * Xl / 3.;
+      aj = (cj.x - (P.es_ref_compat ? 0. : cj.y)) * Xl / 3.;
     }
-    o[rr] = cth * (E[0] - E[1]) / (2. * eps);
-    for (int ss = 0; ss < mdim; ss++)
-      o[3 * mdim + ss * mdim + rr] = (F[0][ss] - F[1][ss]) / (2. * eps);
+    double *o = bond + R * q, *A = J + M2 * (q + i + 1);
+#pragma unroll
+    for (int d = 0; d < MD; d++) {
+      const double f = Y[d] / Yl * wv;
+      o[MD + d] = f * aj;
+      sum[MD + d] += f * ai;
+    }
+#pragma unroll
+    for (int rr = 0; rr < MD; rr++) {
+      double F[2][3], E[2];
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        double um[3] = {uj[0], uj[1], uj[2]}, Z[3], Xm;
+        um[rr] = um[rr] + (w ? -eps : eps);
+        es_geom64<SD>(xi, ui, xj, um, Z, Xm, E[w]);
+        const double Zl = sqrt(Z[0] * Z[0] + Z[1] * Z[1] + Z[2] * Z[2]);
+        const double s =
+            (esqs_t(P, MD, mi, thi, E[w], Xl) + esqs_t(P, MD, mj, thj, E[w], Xl)) * wv;
+        for (int d = 0; d < 3; d++) F[w][d] = (Z[d] / Zl) * s;
+      }
+      const double B = cth * (E[0] - E[1]) / (2. * eps);
+      o[rr] = B;
+      sum[rr] += B;
+#pragma unroll
+      for (int ss = 0; ss < MD; ss++) {
+        const double v = (F[0][ss] - F[1][ss]) / (2. * eps);
+        A[ss * MD + rr] = v;
+        sum[2 * MD + ss * MD + rr] += v;
+      }
+    }
   }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+    for (int d = 0; d < Q; d++) sum[d] += __shfl_xor_sync(0xffffffffu, sum[d], s);
+  if (lane == 0)
+    for (int d = 0; d < Q; d++) sums[Q * i + d] = sum[d];
 }
 
 // Position of the node with original id key in row k (ascending original
@@ -213,39 +238,18 @@ __device__ __forceinline__ int row_find(const int64_t *rowptr, const int *ocols,
   return lo < end && ocols[lo] == key ? (int)(lo - r0) : -1;
 }
 
-// Sums over a row's bonds, in one fixed order: sum B, sum dF/dtheta_i, sum A.
-// A warp per row.
-template <int MD>
-__global__ void __launch_bounds__(128)
-    k_esqs_sums(int64_t n, const int64_t *rowptr, const double *bond, double *sums) {
-  constexpr int R = 3 * MD + MD * MD, Q = 2 * MD + MD * MD;
-  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;
-  const int lane = threadIdx.x & 31;
-  double v[Q] = {};
-  for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += 32) {
-    const double *o = bond + R * q;
-    for (int d = 0; d < MD; d++) v[d] += o[d];
-    for (int d = 0; d < MD + MD * MD; d++) v[MD + d] += o[2 * MD + d];
-  }
-  for (int s = 16; s > 0; s >>= 1)
-    for (int d = 0; d < Q; d++) v[d] += __shfl_xor_sync(0xffffffffu, v[d], s);
-  if (lane == 0)
-    for (int d = 0; d < Q; d++) sums[Q * i + d] = v[d];
-}
-
 // A block of four warps per row node i: lanes over the blocks b (b = 0: i
 // itself, b = 1 + k: the k-th neighbour), warps over the neighbours k whose
 // dilatation u_j moves (the search of j in row k is a chain of loads: one warp
 // per row took 196 us for 1,440 rows, 35 us with four).  full = 0 keeps
 // the (i, rr; j, rr) entries only, as the reference does; full = 1 whole
-// blocks.  Block b of row i is row-major at J[mdim^2 (rowptr[i] + i + b)]; rows
-// and columns of fixed dofs are zero.
+// blocks.  Block b of row i is row-major at J[mdim^2 (rowptr[i] + i + b)], where
+// k_esqs_bonds has left A; rows and columns of fixed dofs are zero.
 template <int MD>
 __global__ void __launch_bounds__(128)
     k_esqs_rows(const DevPtrs D, int full, const int *ocols, const double *bond,
                 const double *sums, double *J) {
-  constexpr int R = 3 * MD + MD * MD, Q = 2 * MD + MD * MD, M2 = MD * MD;
+  constexpr int R = 2 * MD, Q = 2 * MD + MD * MD, M2 = MD * MD;
   __shared__ double part[3][M2][32];
   const int64_t i = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -283,7 +287,7 @@ __global__ void __launch_bounds__(128)
       for (int ss = 0; ss < MD; ss++)
         for (int rr = 0; rr < MD; rr++) {
           const int d = ss * MD + rr;
-          const double own = b == 0 ? -A[d] - G[ss] * C[rr] : o[3 * MD + d] + G[ss] * o[rr];
+          const double own = b == 0 ? -A[d] - G[ss] * C[rr] : blk[d] + G[ss] * o[rr];
           const double v = own + acc[d] + part[0][d][lane] + part[1][d][lane] + part[2][d][lane];
           const bool on = (full || ss == rr) && !dof_fixed(fli, ss, MD) && !dof_fixed(flj, rr, MD);
           blk[d] = on ? v : 0.;
@@ -293,14 +297,11 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Row node and original column id of every directed bond.
-__global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *rows, int *ocols) {
+// Original column id of every directed bond.
+__global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *ocols) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  for (int64_t q = D.rowptr[i]; q < D.rowptr[i + 1]; q++) {
-    rows[q] = (int)i;
-    ocols[q] = D.perm_dev[D.cols[q]];
-  }
+  for (int64_t q = D.rowptr[i]; q < D.rowptr[i + 1]; q++) ocols[q] = D.perm_dev[D.cols[q]];
 }
 
 // ---- BiCGSTAB (van der Vorst 1992) --------------------------------------------
@@ -662,27 +663,21 @@ cudaError_t esqs_residual(const StepParams &P, const DevPtrs &D, int S, int mdim
   return cudaGetLastError();
 }
 
-cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *rows, int *ocols,
-                          cudaStream_t s) {
+cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *ocols, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  k_esqs_topology<<<blocks_of(P.n, 128), 128, 0, s>>>(P.n, D, rows, ocols);
+  k_esqs_topology<<<blocks_of(P.n, 128), 128, 0, s>>>(P.n, D, ocols);
   return cudaGetLastError();
 }
 
 cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim, int full,
-                          const double *u, const double *theta, double eps, int64_t nnz,
-                          const int *rows, const int *ocols, double *bond, double *sums,
-                          double *J, cudaStream_t s) {
+                          const double *u, const double *theta, double eps, const int *ocols,
+                          double *bond, double *sums, double *J, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  if (nnz > 0) {
-    const unsigned g = blocks_of(nnz, 128);
-    (S == 2 ? k_esqs_bonds<2> : k_esqs_bonds<3>)<<<g, 128, 0, s>>>(P, D, mdim, rows, nnz, u, theta,
-                                                                   eps, bond);
-  }
-  (mdim == 1   ? k_esqs_sums<1>
-   : mdim == 2 ? k_esqs_sums<2>
-               : k_esqs_sums<3>)<<<blocks_of(32 * P.n, 128), 128, 0, s>>>(P.n, D.rowptr, bond,
-                                                                          sums);
+  // (a mesh of 1 or 2 dimensions is stored as a 2-D one)
+  (mdim == 3   ? k_esqs_bonds<3, 3>
+   : mdim == 2 ? k_esqs_bonds<2, 2>
+               : k_esqs_bonds<2, 1>)<<<blocks_of(32 * P.n, 128), 128, 0, s>>>(P, D, u, theta, eps,
+                                                                              bond, sums, J);
   (mdim == 1   ? k_esqs_rows<1>
    : mdim == 2 ? k_esqs_rows<2>
                : k_esqs_rows<3>)<<<(unsigned)P.n, 128, 0, s>>>(D, full, ocols, bond, sums, J);

@@ -18,9 +18,9 @@ struct nlm_esqs {
   double *dx = nullptr, *J = nullptr, *part = nullptr, *sc = nullptr;
   BiArgs bi{};
   cudaGraphExec_t bi_graph = nullptr;
-  // Jacobian assembly: per-bond differences, row and original column of a bond
+  // Jacobian assembly: per-bond differences, row sums, original column of a bond
   double *bond = nullptr, *sums = nullptr;
-  int *rows = nullptr, *ocols = nullptr;
+  int *ocols = nullptr;
   std::vector<void *> allocs;
   ~nlm_esqs() {
     if (fd && fd->stream) cudaStreamSynchronize(fd->stream);
@@ -118,11 +118,10 @@ int nlm_esqs_create(const nlm_fd_desc *desc, const nlm_esqs_params *prm, nlm_esq
   if (e == cudaSuccess) e = q->alloc(&bi.sc, 4);
   const size_t md = (size_t)q->mdim;
   if (e == cudaSuccess) e = q->alloc(&q->J, md * md * q->nblocks);
-  if (e == cudaSuccess) e = q->alloc(&q->bond, (3 * md + md * md) * (size_t)h->nnz);
+  if (e == cudaSuccess) e = q->alloc(&q->bond, 2 * md * (size_t)h->nnz);
   if (e == cudaSuccess) e = q->alloc(&q->sums, (2 * md + md * md) * (size_t)h->n);
-  if (e == cudaSuccess) e = q->alloc(&q->rows, (size_t)h->nnz);
   if (e == cudaSuccess) e = q->alloc(&q->ocols, (size_t)h->nnz);
-  if (e == cudaSuccess) e = esqs_topology(h->P, h->D, q->rows, q->ocols, h->stream);
+  if (e == cudaSuccess) e = esqs_topology(h->P, h->D, q->ocols, h->stream);
   if (e == cudaSuccess) e = q->alloc(&q->part, kEsqsDotParts);
   if (e == cudaSuccess) e = q->alloc(&q->sc, 1);
   bi.n = h->n;
@@ -180,7 +179,7 @@ int nlm_esqs_solve(nlm_esqs *q, int nsteps, int *newton_iters, int *lin_iters,
     while (!converged() && it < q->prm.max_iters) {
       // theta is esqs_eval's, at the current u
       cudaError_t e = esqs_jacobian(h->P, h->D, h->S, q->mdim, q->prm.jacobian, u, q->theta, eps,
-                                    h->nnz, q->rows, q->ocols, q->bond, q->sums, q->J, s);
+                                    q->ocols, q->bond, q->sums, q->J, s);
       if (e == cudaSuccess) e = esqs_lin3(q->m, -1., q->res, 0., nullptr, 0., nullptr, q->rhs, s);
       if (e != cudaSuccess) return cuda_fail(e, "quasi-static Jacobian");
       int li = 0;

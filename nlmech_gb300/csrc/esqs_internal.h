@@ -16,16 +16,13 @@ cudaError_t esqs_force(const StepParams &P, const DevPtrs &D, int S, int mdim, c
 // r = f + b on free dofs, 0 on fixed dofs.
 cudaError_t esqs_residual(const StepParams &P, const DevPtrs &D, int S, int mdim,
                           const double *f, const double *b, double *r, cudaStream_t s);
-// rows, ocols: row node and original column id of every directed bond
-cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *rows, int *ocols,
-                          cudaStream_t s);
+// ocols: original column id of every directed bond
+cudaError_t esqs_topology(const StepParams &P, const DevPtrs &D, int *ocols, cudaStream_t s);
 // Jacobian blocks (mdim^2 each, nnz + n of them) at u; theta: the dilatations
-// at u; bond: 3 mdim + mdim^2 doubles per directed bond,
-// sums: 2 mdim + mdim^2 per node
+// at u; bond: 2 mdim doubles per directed bond, sums: 2 mdim + mdim^2 per node
 cudaError_t esqs_jacobian(const StepParams &P, const DevPtrs &D, int S, int mdim, int full,
-                          const double *u, const double *theta, double eps, int64_t nnz,
-                          const int *rows, const int *ocols, double *bond, double *sums,
-                          double *J, cudaStream_t s);
+                          const double *u, const double *theta, double eps, const int *ocols,
+                          double *bond, double *sums, double *J, cudaStream_t s);
 // BiCGSTAB state on the device (sc: slots 0-1 written by the direction launch,
 // 2-3 by the shadow launch, by iteration parity).
 struct BiScal {

@@ -1113,37 +1113,6 @@ __global__ void k_cg32_seed(float *fs, float *pold, int64_t m) {
   if (k == 0) fs[1] = 0.f;
 }
 
-// Bonds of the converged state that exceed the critical strain break.
-template <int DIM>
-__global__ void k_qs_break(const StepParams P, const DevPtrs D, const double *u,
-                           unsigned long long *count) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
-  double xi[3], ui[3];
-  ld_node<DIM>(D.pos64, i, xi);
-  ld_node<DIM>(u, i, ui);
-  const uint8_t fl = D.flags[i];
-  const int64_t r0 = D.rowptr[i], r1 = D.rowptr[i + 1];
-  int newly = 0;
-  for (int64_t q = r0; q < r1; q++) {
-    const int kk = (int)(q - r0);
-    const int64_t w = (int64_t)(kk >> 5) * P.npad + i;
-    const uint32_t word = D.bits[w];
-    if ((word >> (kk & 31)) & 1u) continue;
-    const int j = D.cols[q];
-    if (P.nofail && ((fl & FLAG_NOFAIL) || (D.flags[j] & FLAG_NOFAIL))) continue;
-    double xj[3], uj[3], e[3], r, S, k, ex;
-    ld_node<DIM>(D.pos64, j, xj);
-    ld_node<DIM>(u, j, uj);
-    qs_bond<DIM>(P, xi, ui, xj, uj, D.vol64[j], e, r, S, k, ex);
-    if (P.irrev && dGT(fabs(S), P.fsc * (P.rbar / sqrt(r)))) {
-      D.bits[w] = word | (1u << (kk & 31));
-      newly++;
-    }
-  }
-  if (newly) atomicAdd(count, (unsigned long long)newly);
-}
-
 // u_full (S doubles per node) <-> dof vectors (DIM per node).
 template <int DIM>
 __global__ void k_qs_add(int64_t n, const double *du, double *u) {
@@ -1583,17 +1552,6 @@ cudaError_t qs_add(const StepParams &P, const double *du, double *u, cudaStream_
     k_qs_add<2><<<qblk(P.n), 256, 0, s>>>(P.n, du, u);
   else
     k_qs_add<3><<<qblk(P.n), 256, 0, s>>>(P.n, du, u);
-  return cudaGetLastError();
-}
-
-cudaError_t qs_break(const StepParams &P, const DevPtrs &D, const double *u,
-                     unsigned long long *count, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned long long), s);
-  if (e) return e;
-  if (P.dim == 2)
-    k_qs_break<2><<<qblk(P.n), 256, 0, s>>>(P, D, u, count);
-  else
-    k_qs_break<3><<<qblk(P.n), 256, 0, s>>>(P, D, u, count);
   return cudaGetLastError();
 }
 

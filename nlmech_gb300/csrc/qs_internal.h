@@ -78,7 +78,5 @@ cudaError_t qs_bcdiff(const StepParams &P, const DevPtrs &D, const double *u,
 cudaError_t qs_spmv(const StepParams &P, const DevPtrs &D, const double *blk, const double *dblk,
                     const double *x, double *y, double *part, cudaStream_t s);
 cudaError_t qs_sub(int64_t m, const double *a, const double *b, double *out, cudaStream_t s);
-cudaError_t qs_break(const StepParams &P, const DevPtrs &D, const double *u,
-                     unsigned long long *count, cudaStream_t s);
 
 }  // namespace nlm

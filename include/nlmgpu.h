@@ -70,8 +70,12 @@ enum nlm_decomposition {
   NLM_DECOMP_WARP = 2,    /* one warp per node, CSR bond storage           */
   NLM_DECOMP_THREAD1 = 3, /* one thread per node, one bond per iteration; in
                              FP64: bond geometry recomputed every step instead
-                             of kept in HBM (68 bytes per 2-D bond), slower,
-                             same results                                  */
+                             of kept in HBM (68 bytes per 2-D bond; taken where
+                             it is at most half of what is free, so ask for
+                             THREAD1 where many models share a device), a
+                             quarter of the speed, same results; what
+                             nlm_fd_decomposition gives for an FP64 model that
+                             had no room                                   */
   NLM_DECOMP_TILE = 4,    /* FP32C 2-D RNPBond: 256-node tiles with their
                              halo staged in shared memory, 16-bit
                              tile-local bond ids                           */

@@ -1113,10 +1113,13 @@ int create_model(const nlm_fd_desc *d, nlm_fd **out, bool explicit_steps) {
     *out = nullptr;
     return bail(rc);
   }
-  if (explicit_steps && h->precision == NLM_PREC_FP64 && h->decomp != NLM_DECOMP_THREAD1 &&
-      (rc = build_bond_store64(h))) {
-    *out = nullptr;
-    return bail(rc);
+  if (explicit_steps && h->precision == NLM_PREC_FP64 && h->decomp != NLM_DECOMP_THREAD1) {
+    if ((rc = build_bond_store64(h))) {
+      *out = nullptr;
+      return bail(rc);
+    }
+    // nlm_fd_decomposition tells that there was no room for it
+    if (!h->D.b64_d && !h->D.es64_x) h->decomp = NLM_DECOMP_THREAD1;
   }
   // algorithmic bytes of one step launch (compulsory traffic model)
   {

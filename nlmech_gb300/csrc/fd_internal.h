@@ -62,12 +62,12 @@ struct DevPtrs {
   float2 *es_ab;          // FP32C: t = a |X| + b e coefficients per node
   int *err;               // device error flag
   const int *perm_dev;    // internal -> original node id
-  // time functions of the Displacement_BC sets (as a kernel argument their
-  // 1.3 KB made up half of what a launch carries)
   // batched specimens (FP32C RNPBond): per-slice specimen id, per-specimen
   // FP32 constants (Params32)
   const int *slice_spec;
   const void *qtab;
+  // time functions of the Displacement_BC sets (as a kernel argument their
+  // 1.3 KB made up half of what a launch carries)
   const BCTime *bct;
   // tile store (FP32C 2-D, NLM_DECOMP_TILE): per bond the index of its
   // neighbour in the tile's staged node list (the tile's kTileNodes nodes,

@@ -1128,7 +1128,10 @@ static void qs_force_dim(const StepParams &P, const DevPtrs &D, const double *u,
                          double *blk, double *dblk, bool assemble, unsigned long long *count,
                          cudaStream_t s) {
   if (D.b64_d) {
-    // four lanes per node until one thread per node fills the chip
+    // four lanes per node until one thread per node fills the chip: us per load
+    // step of three evaluations with one / four lanes, 2-D horizon 3h -- 400 nodes
+    // 442 / 331, 10,000: 475 / 428, 40,000: 774 / 696, 90,000: 1149 / 1110, 129,600:
+    // 1445 / 1430, 250,000: 2426 / 2466, 490,000: 4436 / 4442
     const int G = P.n < 131072 ? 4 : 1;
     const unsigned g = (unsigned)((P.n * G + 127) / 128);
     const double ks = P.C * P.beta / P.invF, nib = -1. / P.beta;

@@ -328,7 +328,7 @@ __global__ void k_esqs_topology(int64_t n, const DevPtrs D, int *ocols) {
 
 constexpr int kBiThreads = 64;
 constexpr int kBiTeam = 8;  // lanes per row of J
-constexpr double kBiCancel = 0x1p-10;  // r.r by difference: good to 2^-42 or better
+constexpr double kBiCancel = 0x1p-16;  // r.r by difference: good to 2^-36 or better
 
 // Totals of N partial arrays of gridDim.x entries each, in one fixed order
 // (one warp; lane 0 ends with them).
